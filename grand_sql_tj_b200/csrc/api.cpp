@@ -281,6 +281,7 @@ int tjb::install_plan(tj_ctx *ctx, std::unique_ptr<HpsiPlan> P, uint64_t h,
   if ((rc = ctx->slots.reserve(sizeof(double) * (std::max(P->nslots1, P->nslots2) * BM * BN + 4)))) return rc;
   if ((rc = ctx->scr.reserve(sizeof(double) * (P->scratch_len + 4)))) return rc;
   if ((rc = ctx->counters.reserve(64))) return rc;
+  CK(cudaMemsetAsync(ctx->counters.p, 0, 64, ctx->stream));
   if ((rc = ctx->partials.reserve(sizeof(double) * (std::max(P->tiles2.size(), P->tiles1.size()) + 4096))))
     return rc;
   const double upload_ms = ms_since(t_up) - ozplan_ms;   // host time of the uploads themselves
@@ -425,8 +426,7 @@ int tjb::reset_device_flags(tj_ctx *ctx) {
 int tjb::run_hpsi(tj_ctx *ctx, const double *in, double *out, bool timed) {
   if (ctx->oz) return run_hpsi_oz(ctx, in, out, timed);
   const HpsiPlan &P = *ctx->plan;
-  unsigned int *cnt = (unsigned int *)ctx->counters.p;
-  CK(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned int), ctx->stream));
+  unsigned int *cnt = (unsigned int *)ctx->counters.p;   // zero, and left so by every launch
   if (timed) {
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));

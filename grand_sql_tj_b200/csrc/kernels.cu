@@ -10,18 +10,70 @@
 namespace tjb {
 
 // ------------------------------------------------------------ grouped GEMM
-// One persistent CTA (4 warps) repeatedly takes a 64x64 tile of a cell from a
-// global counter and accumulates sum_t coef_t * op(L_t) * op(R_t) over the
-// cell's tasks with FP64 DMMA (mma.sync m8n8k4).  Operand tiles are staged in
-// shared memory in the layout that keeps the global reads coalesced:
-// [k][m] when op(L) is stored m-contiguous, [m][k] when k-contiguous (same
-// for R), each padded by 4 doubles so the fragment reads are conflict-free.
-constexpr int LDS_KM = BM + 4;   // [k][m] leading dimension
-constexpr int LDS_KN = BN + 4;   // [k][n]
-constexpr int LDS_MK = BK + 4;   // [m][k] and [n][k]
-constexpr int SMEM_L = (BM * LDS_MK > BK * LDS_KM) ? BM * LDS_MK : BK * LDS_KM;
-constexpr int SMEM_R = (BN * LDS_MK > BK * LDS_KN) ? BN * LDS_MK : BK * LDS_KN;
-constexpr int GEMM_THREADS = 128;
+// Persistent CTAs of four multiplying warps and two copying warps take 64x64
+// tiles of cells, the first by their index and the others from a global
+// counter, and accumulate sum_t coef_t * op(L_t) * op(R_t) over the cell's
+// tasks with FP64 DMMA (mma.sync m8n8k4).
+//
+// All tiles of a CTA are one stream of steps of up to GEMM_BK inner-dimension
+// entries, carried through GEMM_STAGES shared-memory stages.  A step takes
+// whatever the next tasks of the tile give, each padded to groups of four
+// entries with its own coefficient: half of the tasks of a superblock have an
+// inner dimension of 13 and less, and a step per task left the cost of a step
+// (its barriers and waits, some 400 cycles) larger than its products.  One
+// copying warp fetches the L operands, the other the R operands, with
+// cp.async, over task and tile borders; stages are handed over by named
+// barriers (hardware barriers, no polling).  Sub-blocks have any leading
+// dimension, so the copies are of single doubles.  A stage holds an operand
+// as [k][i], i the row of op(L) or the column of op(R), at
+// k * 64 + (i ^ f(k)) with f exchanging two bit pairs of k: copies along i,
+// copies along k and fragment reads are all free of bank conflicts without
+// padding.
+//
+// DMMA issues once per 16 cycles and sub-core and reaches 37 TFLOP/s from
+// registers with one warp per sub-core, so a tile costs its DMMAs as long as
+// nothing else is in the multiplying warps' way: the copies' address work is
+// in warps of their own, the loop over a tile's steps is compiled for the
+// warp's number of granules, and of the eight 8-row and eight 8-column
+// granules of a tile only those inside the cell are copied and multiplied,
+// with inner dimensions padded to 4 (the sub-blocks of a superblock fill
+// 64x64x16 tiles to a half at m = 2000 and to a percent at m = 256).
+// Granules go to the warps alternately, so that a part-filled tile still
+// spreads over all four.  Two CTAs per SM, for the registers: held to 128 a
+// thread for more of them, the accumulators are moved about and the kernel
+// takes half as long again.
+//
+// Both launches of the FP64 H*psi of the 4x24 m = 2000 superblock together:
+// 1355 -> 760 us (DMMA pipe 33 -> 60 % on products that count); grand-canonical
+// 4x6 m = 300: 185 -> 80 us; 2x16 ladder m = 256: 55 -> 16 us; one 1024^3
+// block: 18.7 -> 29.4 TFLOP/s.
+constexpr int GEMM_MMA = 128, GEMM_COPY = 64;   // threads that multiply / copy
+constexpr int GEMM_THREADS = GEMM_MMA + GEMM_COPY;
+constexpr int GEMM_BK = 32;                      // inner-dimension entries of a step
+constexpr int GEMM_STAGES = 3;
+constexpr int GEMM_LAG = 1;                      // a step is handed over when this many later ones have been issued
+constexpr int GEMM_STAGE_D = (BM + BN) * GEMM_BK;   // doubles of one stage
+constexpr int GEMM_SMEM = GEMM_STAGES * GEMM_STAGE_D * 8;
+constexpr int GEMM_CTAS = 2;                     // resident per SM
+// named barriers (0 is __syncthreads): stage filled, stage read, next tile
+constexpr int GEMM_FULL = 1, GEMM_EMPTY = GEMM_FULL + GEMM_STAGES, GEMM_NEXT = GEMM_EMPTY + GEMM_STAGES;
+
+// what the multiplying warps learn with a stage
+struct GemmStep {
+  double coef[GEMM_BK / 4];   // of each group of four k
+  int kn;                     // groups of four k
+  int last;                   // 1: the tile's last step, 2: no more steps
+  int nrow, ncol;             // of the tile
+  int tile;                   // index of the tile (its partial sum in dot mode)
+  int pad;
+  Tile tl;                    // set at the last step
+  Cell c;
+};
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
 
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -33,130 +85,334 @@ __device__ __forceinline__ const double *space_base(const GemmParams &p, int sp)
   return sp == SP_OPS ? p.ops : (sp == SP_PSI ? p.psi : p.scr);
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS, 4) grouped_gemm_f64(GemmParams p) {
-  __shared__ __align__(16) double Ls[SMEM_L];
-  __shared__ __align__(16) double Rs[SMEM_R];
-  __shared__ int s_tile;
-  __shared__ double s_red[GEMM_THREADS / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wr = warp >> 1, wc = warp & 1;
+// the place of k in the swizzle of a stage: its low two bit pairs exchanged
+__device__ __forceinline__ int gemm_f(int k) { return ((k & 3) << 2) | (k >> 2 & 3); }
 
+// 8 bytes from global to shared memory; n = 0: zeros, src not read
+__device__ __forceinline__ void cp_async8z(uint32_t dst, const double *src, int n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// One operand's k in [0, kv) into groups g, g + 1, ... of a stage, by one
+// warp, element (i, k) at src[k * ld + i]: the lanes along i (2^LG < 32 of
+// them: 32 >> LG k at a time).  Rows past n are left as they are (they meet
+// only output rows past the cell); the last group is filled up with zeros.
+template <int LG>
+__device__ __forceinline__ void gemm_copy_i(uint32_t dst, const double *src, int ld, int n, int g, int kv) {
+  constexpr int ST = 32 >> LG;   // k apart of a lane's copies
+  const int lane = threadIdx.x & 31, i = lane & ((1 << LG) - 1), kb = lane >> LG;
+  if (i >= n) return;
+  const double *s = src + (int64_t)kb * ld + i;
+  const int64_t st = (int64_t)ST * ld;
+  const bool in2 = LG == 5 && i + 32 < n;
+  uint32_t d = dst + (uint32_t)((4 * g + kb) * BM + (i ^ (kb << 2))) * 8u;
+  int k = 0;
+#pragma unroll 2
+  for (; k + 4 <= kv; k += 4, ++g, d += 4 * BM * 8) {
+    const uint32_t x = d ^ (uint32_t)((g & 3) * 8);
+#pragma unroll
+    for (int j = 0; j < 4; j += ST) {
+      cp_async8((x ^ (uint32_t)(j * 32)) + j * BM * 8, s);
+      if (in2) cp_async8((x ^ (uint32_t)(j * 32)) + j * BM * 8 + 256, s + 32);
+      s += st;
+    }
+  }
+  if (k < kv) {
+    const uint32_t x = d ^ (uint32_t)((g & 3) * 8);
+#pragma unroll
+    for (int j = 0; j < 4; j += ST) {
+      const int bytes = k + kb + j < kv ? 8 : 0;
+      cp_async8z((x ^ (uint32_t)(j * 32)) + j * BM * 8, s, bytes);
+      if (in2) cp_async8z((x ^ (uint32_t)(j * 32)) + j * BM * 8 + 256, s + 32, bytes);
+      s += st;
+    }
+  }
+}
+// Element (i, k) at src[i * ld + k]: the lanes along k, 2^LK of them, 32 >> LK
+// rows at a time.
+template <int LK>
+__device__ __forceinline__ void gemm_copy_k(uint32_t dst, const double *src, int ld, int n, int g, int kv) {
+  constexpr int R = 32 >> LK;
+  const int lane = threadIdx.x & 31, k = lane & ((1 << LK) - 1), ib = lane >> LK, at = 4 * g + k;
+  if (k >= ((kv + 3) & ~3)) return;
+  const double *s = src + (int64_t)ib * ld + k;
+  const int64_t st = R * (int64_t)ld;
+  const uint32_t d0 = dst + (uint32_t)(at * BM) * 8u;
+  const uint32_t f = (uint32_t)gemm_f(at);
+  const int bytes = k < kv ? 8 : 0;
+#pragma unroll 4
+  for (int i = ib; i < n; i += R, s += st) cp_async8z(d0 + ((uint32_t)i ^ f) * 8u, s, bytes);
+}
+
+// The warp's MM x NN granules of one step; la, lb: the lane's places in
+// granule 0 of the two operands for each group kk of four k; the warp's
+// granules are 16 entries apart.
+template <int MM, int NN>
+__device__ __forceinline__ void gemm_mma(double (&acc)[4][4][2], const double *st, const int (&la)[4],
+                                         const int (&lb)[4], const double *coef, int kn) {
+  auto load = [&](int kk, double (&a)[MM], double (&b)[NN]) {
+    const double cf = coef[kk];
+#pragma unroll
+    for (int mi = 0; mi < MM; ++mi) a[mi] = cf * st[la[kk] + mi * 16];
+#pragma unroll
+    for (int ni = 0; ni < NN; ++ni) b[ni] = st[lb[kk] + ni * 16];
+  };
+  auto mul = [&](const double (&a)[MM], const double (&b)[NN]) {
+#pragma unroll
+    for (int mi = 0; mi < MM; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < NN; ++ni) dmma_8x8x4(acc[mi][ni], a[mi], b[ni]);
+  };
+  // the next group's fragments are read under this group's products
+  for (; kn >= 4; kn -= 4, st += 16 * BM, coef += 4) {
+    double a[2][MM], b[2][NN];
+    load(0, a[0], b[0]);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      if (kk < 3) load(kk + 1, a[(kk + 1) & 1], b[(kk + 1) & 1]);
+      mul(a[kk & 1], b[kk & 1]);
+    }
+  }
+#pragma unroll
+  for (int kk = 0; kk < 3; ++kk) {
+    if (kk >= kn) break;
+    double a[MM], b[NN];
+    load(kk, a, b);
+    mul(a, b);
+  }
+}
+
+// The steps of one tile for a warp that holds MM x NN of its granules, from
+// the one in `stage` (filled) to the last, which is left to the caller.
+template <int MM, int NN>
+__device__ __forceinline__ void gemm_tile(double (&acc)[4][4][2], const double *gsm, const GemmStep *step, int &stage,
+                                          const int (&la)[4], const int (&lb)[4]) {
   for (;;) {
-    if (tid == 0) s_tile = (int)atomicAdd(p.counter, 1u);
-    __syncthreads();
-    const int t = s_tile;
-    __syncthreads();
-    if (t >= p.ntiles) return;
+    const GemmStep &s = step[stage];
+    const int last = s.last, kn = s.kn;
+    if (MM > 0) gemm_mma<MM == 0 ? 1 : MM, NN == 0 ? 1 : NN>(acc, gsm + stage * GEMM_STAGE_D, la, lb, s.coef, kn);
+    if (last) return;
+    bar_arrive(GEMM_EMPTY + stage, GEMM_THREADS);
+    stage = stage == GEMM_STAGES - 1 ? 0 : stage + 1;
+    bar_sync(GEMM_FULL + stage, GEMM_THREADS);
+  }
+}
+
+// The copying warps: warp 0 of them the L operands and the steps' records,
+// warp 1 the R operands.
+__device__ __forceinline__ void gemm_copy_stream(const GemmParams &p, uint32_t sm0, GemmStep *step, int *s_next) {
+  const int lane = threadIdx.x & 31;
+  const bool left = threadIdx.x - GEMM_MMA < 32;
+  int count = 0, stage = 0;   // steps issued, the next one's stage
+  auto hand_over = [&](int n) {   // step n is in shared memory
+    bar_arrive(GEMM_FULL + n % GEMM_STAGES, GEMM_THREADS);
+  };
+  auto acquire = [&]() {
+    if (count >= GEMM_STAGES) bar_sync(GEMM_EMPTY + stage, GEMM_THREADS);
+  };
+  auto issued = [&]() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (count >= GEMM_LAG) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(GEMM_LAG) : "memory");
+      hand_over(count - GEMM_LAG);
+    }
+    ++count;
+    stage = stage == GEMM_STAGES - 1 ? 0 : stage + 1;
+  };
+  for (int t = blockIdx.x; t < p.ntiles;) {
+    // the tile after this one; the CTAs fetch ntiles numbers in all, so the
+    // counter has wrapped to 0 when the launch ends
+    unsigned nxt = 0;
+    if (left && lane == 0) nxt = atomicInc(p.counter, (unsigned)p.ntiles - 1u);
     const Tile tl = p.tiles[t];
     const Cell c = p.cells[tl.cell];
-
-    double acc[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    for (int ti = tl.tb; ti < tl.te; ++ti) {
-      const Task tk = p.tasks[ti];
-      const double *__restrict__ Lb = space_base(p, tk.L.space) + tk.L.off;
-      const double *__restrict__ Rb = space_base(p, tk.R.space) + tk.R.off;
-      const int ldl = tk.L.ld, ldr = tk.R.ld, K = tk.K;
-      const bool lt = tk.L.trans != 0, rt = tk.R.trans != 0;
-      const double coef = tk.coef;
-      const int lsr = lt ? LDS_MK : 1, lsk = lt ? 1 : LDS_KM;
-      const int rsn = rt ? 1 : LDS_MK, rsk = rt ? LDS_KN : 1;
-      for (int k0 = 0; k0 < K; k0 += BK) {
-        if (!lt) {
-          const int r = tid & 63, kb = tid >> 6, gr = tl.row0 + r;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int k = kb + 2 * j, gk = k0 + k;
-            double v = 0.0;
-            if (gr < c.M && gk < K) v = coef * Lb[(int64_t)gk * ldl + gr];
-            Ls[k * LDS_KM + r] = v;
-          }
-        } else {
-          const int k = tid & 15, rb = tid >> 4, gk = k0 + k;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int r = rb + 8 * j, gr = tl.row0 + r;
-            double v = 0.0;
-            if (gr < c.M && gk < K) v = coef * Lb[(int64_t)gr * ldl + gk];
-            Ls[r * LDS_MK + k] = v;
-          }
+    const int nrow = min(BM, c.M - tl.row0), ncol = min(BN, c.N - tl.col0);
+    const int n = left ? nrow : ncol, at = left ? tl.row0 : tl.col0;
+    const int lg = n > 16 ? 5 : n > 8 ? 4 : 3;
+    int g = GEMM_BK / 4;   // groups of the open stage in use; all: none is open
+    bool open = false;
+    auto begin = [&]() {
+      acquire();
+      g = 0;
+      open = true;
+    };
+    auto finish = [&](int last) {
+      if (left && lane == 0) {
+        GemmStep &s = step[stage];
+        s.kn = g;
+        s.last = last;
+        s.nrow = nrow;
+        s.ncol = ncol;
+        if (last) {
+          s.tile = t;
+          s.tl = tl;
+          s.c = c;
         }
-        if (!rt) {
-          const int k = tid & 15, nb = tid >> 4, gk = k0 + k;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int n = nb + 8 * j, gn = tl.col0 + n;
-            double v = 0.0;
-            if (gn < c.N && gk < K) v = Rb[(int64_t)gn * ldr + gk];
-            Rs[n * LDS_MK + k] = v;
+      }
+      issued();
+    };
+    for (int tb = tl.tb; tb < tl.te; tb += 32) {
+      // one task per lane, handed round by shuffles
+      Operand op = Operand{0, 0, 0, 0, 0};
+      double co = 0.0;
+      int Kl = 0;
+      if (tb + lane < tl.te) {
+        const Task *tk = p.tasks + tb + lane;
+        op = left ? tk->L : tk->R;
+        co = tk->coef;
+        Kl = tk->K;
+      }
+      const int nt = min(32, tl.te - tb);
+      for (int q = 0; q < nt; ++q) {
+        const int K = __shfl_sync(0xffffffffu, Kl, q), ld = __shfl_sync(0xffffffffu, op.ld, q);
+        const int fl = __shfl_sync(0xffffffffu, (int)op.space | (int)op.trans << 8, q);
+        const double *src = space_base(p, fl & 255) + __shfl_sync(0xffffffffu, op.off, q);
+        const bool kmajor = left == (fl >> 8 != 0);   // k runs along the stored columns
+        src += kmajor ? (int64_t)at * ld : at;
+        const double coef = __shfl_sync(0xffffffffu, co, q);
+        for (int k0 = 0; k0 < K;) {
+          if (g == GEMM_BK / 4) {
+            if (open) finish(0);
+            begin();
           }
-        } else {
-          const int n = tid & 63, kb = tid >> 6, gn = tl.col0 + n;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int k = kb + 2 * j, gk = k0 + k;
-            double v = 0.0;
-            if (gn < c.N && gk < K) v = Rb[(int64_t)gk * ldr + gn];
-            Rs[k * LDS_KN + n] = v;
-          }
+          const int kv = min(K - k0, GEMM_BK - 4 * g), kp = (kv + 3) & ~3;   // kp: in whole groups
+          const uint32_t d = sm0 + (uint32_t)(stage * GEMM_STAGE_D + (left ? 0 : BM * GEMM_BK)) * 8u;
+          if (kmajor) {
+            if (kp > 16)
+              gemm_copy_k<5>(d, src, ld, n, g, kv);
+            else if (kp > 8)
+              gemm_copy_k<4>(d, src, ld, n, g, kv);
+            else if (kp > 4)
+              gemm_copy_k<3>(d, src, ld, n, g, kv);
+            else
+              gemm_copy_k<2>(d, src, ld, n, g, kv);
+          } else if (lg == 5)
+            gemm_copy_i<5>(d, src, ld, n, g, kv);
+          else if (lg == 4)
+            gemm_copy_i<4>(d, src, ld, n, g, kv);
+          else
+            gemm_copy_i<3>(d, src, ld, n, g, kv);
+          if (left && lane < kp >> 2) step[stage].coef[g + lane] = coef;
+          src += kmajor ? kv : (int64_t)kv * ld;
+          k0 += kv;
+          g += kp >> 2;
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK / 4; ++kk) {
-          const int k = kk * 4 + (lane & 3);
-          double a[4], b[4];
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi) a[mi] = Ls[(wr * 32 + mi * 8 + (lane >> 2)) * lsr + k * lsk];
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) b[ni] = Rs[(wc * 32 + ni * 8 + (lane >> 2)) * rsn + k * rsk];
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma_8x8x4(acc[mi][ni], a[mi], b[ni]);
-        }
-        __syncthreads();
       }
     }
+    if (!open) begin();   // no task: an empty step
+    finish(1);
+    if (left && lane == 0) *s_next = (int)(nxt + gridDim.x);
+    bar_sync(GEMM_NEXT, GEMM_COPY);
+    t = *s_next;
+    bar_sync(GEMM_NEXT, GEMM_COPY);
+  }
+  acquire();
+  if (left && lane == 0) step[stage].last = 2;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int n = count > GEMM_LAG ? count - GEMM_LAG : 0; n <= count; ++n) hand_over(n);
+  // every barrier a stage's readers arrive at is completed before the exit
+  for (int n = count >= GEMM_STAGES ? count - GEMM_STAGES + 1 : 0; n < count; ++n)
+    bar_sync(GEMM_EMPTY + n % GEMM_STAGES, GEMM_THREADS);
+}
 
-    double local = 0.0;
+__global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS) grouped_gemm_f64(GemmParams p) {
+  extern __shared__ __align__(128) double gsm[];
+  __shared__ GemmStep step[GEMM_STAGES];
+  __shared__ int s_next;
+  __shared__ double s_red[GEMM_MMA / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  static_assert(BM == 64 && BN == 64 && GEMM_BK == 32, "layout of the stages");
+  if (tid >= GEMM_MMA) {
+    gemm_copy_stream(p, (uint32_t)__cvta_generic_to_shared(gsm), step, &s_next);
+    return;
+  }
+  const int wr = warp >> 1, wc = warp & 1;
+  int la[4], lb[4];   // gemm_mma's places within a stage
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+  for (int kk = 0; kk < 4; ++kk) {
+    const int k = 4 * kk + (lane & 3);
+    la[kk] = k * BM + ((wr * 8 + (lane >> 2)) ^ gemm_f(k));
+    lb[kk] = BM * GEMM_BK + k * BN + ((wc * 8 + (lane >> 2)) ^ gemm_f(k));
+  }
+  // thread's entries of a tile: 16 mi + er, 16 ni + ec + e
+  const int er = wr * 8 + (lane >> 2), ec = wc * 8 + 2 * (lane & 3);
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int stage = 0;; stage = stage == GEMM_STAGES - 1 ? 0 : stage + 1) {
+    bar_sync(GEMM_FULL + stage, GEMM_THREADS);
+    if (step[stage].last == 2) break;
+    const int nrow = step[stage].nrow, ncol = step[stage].ncol;
+    // this warp's granules: rows wr, wr + 2, ..., columns wc, wc + 2, ...
+    const int mym = (((nrow + 7) >> 3) + 1 - wr) >> 1, myn = (((ncol + 7) >> 3) + 1 - wc) >> 1;
+#define GEMM_CASE(MM, NN) case MM * 8 + NN: gemm_tile<MM, NN>(acc, gsm, step, stage, la, lb); break
+    switch (mym * 8 + myn) {
+      GEMM_CASE(1, 1); GEMM_CASE(1, 2); GEMM_CASE(1, 3); GEMM_CASE(1, 4);
+      GEMM_CASE(2, 1); GEMM_CASE(2, 2); GEMM_CASE(2, 3); GEMM_CASE(2, 4);
+      GEMM_CASE(3, 1); GEMM_CASE(3, 2); GEMM_CASE(3, 3); GEMM_CASE(3, 4);
+      GEMM_CASE(4, 1); GEMM_CASE(4, 2); GEMM_CASE(4, 3); GEMM_CASE(4, 4);
+      default: gemm_tile<0, 0>(acc, gsm, step, stage, la, lb); break;   // no granule of the tile is this warp's
+    }
+#undef GEMM_CASE
+    const GemmStep &sp = step[stage];
+    const Tile tl = sp.tl;
+    const int64_t c_off = sp.c.off;
+    const int c_ld = sp.c.ld, tile = sp.tile;
+    bar_arrive(GEMM_EMPTY + stage, GEMM_THREADS);
+    for (int tj = tl.ab; tj < tl.ae; ++tj) {
+      const Task ax = p.tasks[tj];
+      const double *x = space_base(p, ax.L.space) + ax.L.off + (int64_t)(tl.col0 + ec) * ax.L.ld + tl.row0 + er;
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int r = tl.row0 + wr * 32 + mi * 8 + (lane >> 2);
-          const int n = tl.col0 + wc * 32 + ni * 8 + 2 * (lane & 3) + e;
-          if (r < c.M && n < c.N) {
-            double v = acc[mi][ni][e];
-            for (int tj = tl.ab; tj < tl.ae; ++tj) {
-              const Task &ax = p.tasks[tj];
-              v += ax.coef * space_base(p, ax.L.space)[ax.L.off + (int64_t)n * ax.L.ld + r];
-            }
-            const int64_t o = c.off + (int64_t)n * c.ld + r;
-            if (p.dot_mode)
-              local += v * p.dot_with[o];
-            else if (tl.slot < 0)
-              p.out[o] = v;
-            else
-              p.slots[(int64_t)tl.slot * (BM * BN) + (n - tl.col0) * BM + (r - tl.row0)] = v;
-          }
+          const double *xc = x + (int64_t)(ni * 16 + e) * ax.L.ld;
+          if (ni * 16 + ec + e < ncol)
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi)
+              if (mi * 16 + er < nrow) acc[mi][ni][e] += ax.coef * xc[mi * 16];
         }
-    if (p.dot_mode) {
+    }
+    const bool dot = p.dot_mode != 0, slot = !dot && tl.slot >= 0;
+    const int64_t o0 = slot ? (int64_t)tl.slot * (BM * BN) + ec * BM + er
+                            : c_off + (int64_t)(tl.col0 + ec) * c_ld + tl.row0 + er;
+    const int old = slot ? BM : c_ld;
+    double *o = (slot ? p.slots : p.out) + o0;   // dot mode: not written
+    double local = 0.0;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (ni * 16 + ec + e < ncol) {
+          const int64_t oc = (int64_t)(ni * 16 + e) * old;
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi)
+            if (mi * 16 + er < nrow) {
+              if (dot)
+                local += acc[mi][ni][e] * p.dot_with[o0 + oc + mi * 16];
+              else
+                o[oc + mi * 16] = acc[mi][ni][e];
+            }
+        }
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) acc[mi][ni][e] = 0.0;
+      }
+    if (dot) {
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1) local += __shfl_down_sync(0xffffffffu, local, s);
       if (lane == 0) s_red[warp] = local;
-      __syncthreads();
+      bar_sync(GEMM_NEXT + 1, GEMM_MMA);
       if (tid == 0) {
         double tot = 0.0;
-        for (int w = 0; w < GEMM_THREADS / 32; ++w) tot += s_red[w];
-        p.partials[t] = tot;
+        for (int w = 0; w < GEMM_MMA / 32; ++w) tot += s_red[w];
+        p.partials[tile] = tot;
       }
-      __syncthreads();
+      bar_sync(GEMM_NEXT + 1, GEMM_MMA);
     }
   }
 }
@@ -165,36 +421,53 @@ int grouped_gemm_grid(int ntiles, int ctas_per_sm) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int g = sms * std::min(4, std::max(1, ctas_per_sm));
+  int g = sms * std::min(GEMM_CTAS, std::max(1, ctas_per_sm));
   return ntiles < g ? (ntiles > 0 ? ntiles : 1) : g;
 }
 
 void launch_grouped_gemm(const GemmParams &p, int grid, cudaStream_t s) {
   if (p.ntiles <= 0) return;
-  grouped_gemm_f64<<<grid, GEMM_THREADS, 0, s>>>(p);
+  // the attribute belongs to the device's context: set at every launch
+  cudaFuncSetAttribute(grouped_gemm_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+  grouped_gemm_f64<<<grid, GEMM_THREADS, GEMM_SMEM, s>>>(p);
 }
 
-// One CTA per split tile: the slots are added in slot order, so the result
-// does not depend on which items finished first.
-__global__ void reduce_slots_kernel(GemmParams p, const Reduce *red) {
+// Four CTAs per split tile, 16 columns each, one row of four columns a thread:
+// the slots are added in slot order, so the result does not depend on which
+// items finished first; the slots of four columns are in flight together (one
+// CTA per tile and one load at a time took 45 us of the 1.4 ms FP64 H*psi of
+// the 4x24 m = 2000 superblock, 619 tiles).
+__global__ void __launch_bounds__(256) reduce_slots_kernel(GemmParams p, const Reduce *red) {
   const Reduce rd = red[blockIdx.x];
   const Cell c = p.cells[rd.cell];
   const int rows = min(BM, c.M - rd.row0), cols = min(BN, c.N - rd.col0);
-  for (int idx = threadIdx.x; idx < rows * cols; idx += blockDim.x) {
-    const int r = idx % rows, n = idx / rows;
-    double v = 0.0;
-    for (int k = 0; k < rd.nslot; ++k) v += p.slots[(int64_t)(rd.slot0 + k) * (BM * BN) + n * BM + r];
-    const int gr = rd.row0 + r, gn = rd.col0 + n;
-    for (int tj = rd.ab; tj < rd.ae; ++tj) {
-      const Task &ax = p.tasks[tj];
-      v += ax.coef * space_base(p, ax.L.space)[ax.L.off + (int64_t)gn * ax.L.ld + gr];
-    }
-    p.out[c.off + (int64_t)gn * c.ld + gr] = v;
+  const int r = threadIdx.x & (BM - 1), n0 = blockIdx.y * (BN / 4) + threadIdx.x / BM;
+  constexpr int Q = BN / 16, DN = 256 / BM;   // columns of a thread, DN apart
+  if (r >= rows || n0 >= cols) return;
+  double v[Q];
+  const double *s = p.slots + (int64_t)rd.slot0 * (BM * BN) + n0 * BM + r;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) v[q] = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < rd.nslot; ++k, s += BM * BN)
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (n0 + q * DN < cols) v[q] += s[q * DN * BM];
+  for (int tj = rd.ab; tj < rd.ae; ++tj) {
+    const Task ax = p.tasks[tj];
+    const double *x = space_base(p, ax.L.space) + ax.L.off + (int64_t)(rd.col0 + n0) * ax.L.ld + rd.row0 + r;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (n0 + q * DN < cols) v[q] += ax.coef * x[(int64_t)(q * DN) * ax.L.ld];
   }
+  double *o = p.out + c.off + (int64_t)(rd.col0 + n0) * c.ld + rd.row0 + r;
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (n0 + q * DN < cols) o[(int64_t)(q * DN) * c.ld] = v[q];
 }
 
 void launch_reduce(const GemmParams &p, const Reduce *red, int nred, cudaStream_t s) {
-  if (nred > 0) reduce_slots_kernel<<<nred, 256, 0, s>>>(p, red);
+  if (nred > 0) reduce_slots_kernel<<<dim3(nred, 4), 256, 0, s>>>(p, red);
 }
 
 // ------------------------------------------------------------------ merges

@@ -16,7 +16,7 @@ struct GemmParams {
   const Task *tasks;
   const Tile *tiles;
   int ntiles;
-  unsigned int *counter;   // dynamic tile counter (zeroed before launch)
+  unsigned int *counter;   // dynamic tile counter (zero before the launch, zero again after it)
   double *partials;        // dot mode: one partial sum per work item
   double *slots;           // partial tiles of split cells, BM*BN doubles per slot
   const double *dot_with;  // dot mode: vector the result is dotted with (same layout as out)

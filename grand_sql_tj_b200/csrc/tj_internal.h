@@ -97,7 +97,7 @@ struct HpsiPlan {
 };
 
 // Tile shape of the grouped FP64 kernel.
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int BM = 64, BN = 64;
 
 // Tiling and scheduling choices the autotuner searches (defaults: the values
 // set by hand for the 4x24 m = 2000 superblock).
