@@ -15,11 +15,12 @@
 // Sturm-count multisection (one warp per eigenvalue), the host selects the
 // kept states exactly as den_mat.f90 does, and only the kept eigenvectors
 // are computed: inverse iteration on the tridiagonal matrix (one thread per
-// vector), Gram-Schmidt orthonormalisation inside each kept block (one CTA,
-// or a cluster for large blocks), and the back-transformation by the stored
-// reflectors, written straight into the truncation operator's layout, which
-// stays on the device until the second call of the two-call protocol copies
-// it out.  Everything is FP64.
+// vector), Gram-Schmidt orthonormalisation inside each kept block (by two
+// matrix products for the vectors that inverse iteration left nearly
+// orthogonal, vector by vector for the others), and the back-transformation by
+// blocks of the stored reflectors, written straight into the truncation
+// operator's layout, which stays on the device until the second call of the
+// two-call protocol copies it out.  Everything is FP64.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -78,23 +79,60 @@ __device__ __forceinline__ double block_sum(double x, double *red) {
 // p = A v of step k+1, so each step reads and writes the trailing block once.
 // One CTA per sector (tridiag_one) or one cluster per large sector
 // (tridiag_coop).
-__device__ __forceinline__ void tridiag_info(int s, int n, const double *d, const double *e, double *info) {
+// The power of two that scales T's largest row sum tnorm into [1/2, 1); 1 where
+// T is zero (or out of range).
+__device__ __forceinline__ double tridiag_scale(double tnorm) {
+  const int te = __double2hiint(tnorm) >> 20 & 2047;
+  return te > 0 && te < 2045 ? __hiloint2double((2045 - te) << 20, 0) : 1.0;
+}
+
+// By all threads of one CTA: info, and the scaled diagonal ds and squared
+// off-diagonal e2 that the Sturm counts read.  red: 48 doubles.
+__device__ void tridiag_info(int s, int n, const double *d, const double *e, double *info, double *ds, double *e2,
+                             double *red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double gl = 1e308, gu = -1e308, emax2 = 0.0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double el = i > 0 ? fabs(e[i - 1]) : 0.0, er = i + 1 < n ? fabs(e[i]) : 0.0;
     gl = fmin(gl, d[i] - el - er);
     gu = fmax(gu, d[i] + el + er);
     if (i + 1 < n) emax2 = fmax(emax2, e[i] * e[i]);
   }
-  info[4 * s + 0] = gl;
-  info[4 * s + 1] = gu;
-  info[4 * s + 2] = fmax(fabs(gl), fabs(gu));
-  info[4 * s + 3] = EIG_SAFMIN * fmax(1.0, emax2);
+  for (int o = 16; o > 0; o >>= 1) {
+    gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
+    gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
+    emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
+  }
+  __syncthreads();
+  if (lane == 0) {
+    red[warp] = gl;
+    red[16 + warp] = gu;
+    red[32 + warp] = emax2;
+  }
+  __syncthreads();
+  for (int w = 0; w < nw; ++w) {
+    gl = fmin(gl, red[w]);
+    gu = fmax(gu, red[16 + w]);
+    emax2 = fmax(emax2, red[32 + w]);
+  }
+  const double tnorm = fmax(fabs(gl), fabs(gu)), sc = tridiag_scale(tnorm);
+  if (threadIdx.x == 0) {
+    info[4 * s + 0] = gl;
+    info[4 * s + 1] = gu;
+    info[4 * s + 2] = tnorm;
+    info[4 * s + 3] = EIG_SAFMIN * fmax(1.0, emax2);
+  }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    ds[i] = d[i] * sc;
+    const double es = i + 1 < n ? e[i] * sc : 0.0;
+    e2[i] = es * es;
+  }
 }
+static_assert(EIG_THREADS <= 512, "tridiag_info's scratch");
 
 __device__ void tridiag_one(int s, double *Aall, const int64_t *off, const int *dims, const int64_t *eoff,
-                            double *dall, double *eall, double *tauall, double *info, double *sm, double *red,
-                            double &sh_tau, double &sh_scl) {
+                            double *dall, double *eall, double *tauall, double *info, double *dsall, double *e2all,
+                            double *sm, double *red, double &sh_tau, double &sh_scl) {
   const int n = dims[s], tid = threadIdx.x, nt = blockDim.x;
   double *A = Aall + off[s];
   double *d = dall + eoff[s], *e = eall + eoff[s], *tau = tauall + eoff[s];
@@ -198,8 +236,9 @@ __device__ void tridiag_one(int s, double *Aall, const int64_t *off, const int *
   if (tid == 0) {
     d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
     if (n >= 1) tau[n - 1] = 0.0;
-    tridiag_info(s, n, d, e, info);
   }
+  __syncthreads();
+  tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red);
 }
 
 // Sum of one value per thread over the block with one barrier: each warp's
@@ -237,7 +276,8 @@ __device__ __forceinline__ double block_sum1(double x, double *red, int &half) {
 template <int CL>
 __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aall, const int64_t *off,
                              const int *dims, const int64_t *eoff, double *dall, double *eall, double *tauall,
-                             double *info, double *sm, int64_t smem_doubles, double *red2, double *pvs) {
+                             double *info, double *dsall, double *e2all, double *sm, int64_t smem_doubles, double *red2,
+                             double *pvs) {
   const int n = dims[s], tid = threadIdx.x, nt = blockDim.x;
   double *A = Aall + off[s];
   double *d = dall + eoff[s], *e = eall + eoff[s], *tau = tauall + eoff[s];
@@ -425,10 +465,13 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     d[n - 1] = sl[(int64_t)((n - 1 - myr0) / CL) * mres + (n - 1 - kr1)];
   __threadfence();
   cl.sync();   // the last parts are read; every owner's writes are visible
-  if (rank == 0 && tid == 0) {
-    if (!last_in_slice) d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
-    tau[n - 1] = 0.0;
-    tridiag_info(s, n, d, e, info);
+  if (rank == 0) {
+    if (tid == 0) {
+      if (!last_in_slice) d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
+      tau[n - 1] = 0.0;
+    }
+    __syncthreads();
+    tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red2);
   }
 }
 
@@ -440,7 +483,8 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
     tridiag_kernel(double *Aall, const int64_t *off, const int *dims, const int64_t *eoff, const int *tsec,
-                   const int *tbig, double *dall, double *eall, double *tauall, double *info, int64_t smem_doubles) {
+                   const int *tbig, double *dall, double *eall, double *tauall, double *info, double *dsall, double *e2all,
+                   int64_t smem_doubles) {
   extern __shared__ double sm[];
   __shared__ double red[64];
   __shared__ double sh_tau, sh_scl, sh_pvs[16];
@@ -448,25 +492,64 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
   const int b = blockIdx.x / CL, rank = (int)cl.block_rank();
   const int s = tsec[blockIdx.x];
   if (tbig[b]) {
-    tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, info, sm, smem_doubles, red, sh_pvs);
+    tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, sm, smem_doubles, red,
+                     sh_pvs);
   } else if (s >= 0 && dims[s] > 0) {
-    tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, sm, red, sh_tau, sh_scl);
+    tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, sm, red, sh_tau, sh_scl);
   }
 }
 
-// Number of eigenvalues of T below x: the negative LDL^T pivots of T - x I
-// (pivots below pivmin in size are replaced by -pivmin, as LAPACK's dstebz
-// does).
-__device__ __forceinline__ int sturm1(const double *d, const double *e, int n, double pivmin, double x) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = (d[i] - x) - e[i - 1] * e[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += q < 0.0;
+// Number of eigenvalues of the scaled T (diagonal ds, squared off-diagonal e2)
+// below x: the sign changes along the leading principal minors of T - x I,
+// p_{i+1} = (d_i - x) p_i - e_{i-1}^2 p_{i-1}.  The pivots of LDL^T, the ratios
+// of consecutive minors, would cost a division a step; the minors take three
+// operations and a rescaling by a power of two every eight steps.  A zero
+// minor between others needs no care (its neighbours have opposite signs, so
+// either sign of it makes one change); only where eight steps shrink the
+// minors below 2^-500 (a zero pivot at a zero off-diagonal, or entries far
+// under the accuracy asked for) are they repeated with every pivot below 2^-60
+// taken as -2^-60, as LAPACK's dstebz does with its pivmin.
+__device__ __forceinline__ int sturm1(const double *__restrict__ ds, const double *__restrict__ e2, int n, double x) {
+  double p0 = 1.0, p1 = ds[0] - x;
+  if (fabs(p1) < 0x1p-60) p1 = -0x1p-60;
+  int c = __double2hiint(p1) >> 31;   // minus the count
+  auto step = [&](double di, double ei, bool careful) {
+    double p = fma(di - x, p1, -(ei * p0));
+    // |p| < 2^-60 |p1| by the exponents
+    if (careful && (__double2hiint(p) & 0x7ff00000) + (60 << 20) < (__double2hiint(p1) & 0x7ff00000)) p = -0x1p-60 * p1;
+    c += (__double2hiint(p) ^ __double2hiint(p1)) >> 31;
+    p0 = p1;
+    p1 = p;
+  };
+  // the larger exponent of the two last minors
+  auto expo = [&]() { return max(__double2hiint(p0) >> 20 & 2047, __double2hiint(p1) >> 20 & 2047); };
+  int i = 1;
+  for (; i + 8 <= n; i += 8) {
+    double dv[8], ev[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      dv[u] = ds[i + u];
+      ev[u] = e2[i + u - 1];
+    }
+    const double b0 = p0, b1 = p1;
+    const int bc = c;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) step(dv[u], ev[u], false);
+    if (expo() < 1023 - 500) {
+      p0 = b0;
+      p1 = b1;
+      c = bc;
+#pragma unroll 1
+      for (int u = 0; u < 8; ++u) step(ds[i + u], e2[i + u - 1], true);
+    }
+    // the larger of the two to about one
+    const double f = __hiloint2double(min(max(2046 - expo(), 1), 2045) << 20, 0);
+    p0 *= f;
+    p1 *= f;
   }
-  return c;
+#pragma unroll 1
+  for (; i < n; ++i) step(ds[i], e2[i - 1], true);
+  return -c;
 }
 
 // Eigenvalue k (ascending) of every sector, one warp each: the interval
@@ -476,21 +559,24 @@ __device__ __forceinline__ int sturm1(const double *d, const double *e, int n, d
 // and the first above it, until it is below 2 eps max(|lo|, |hi|) or
 // eps ||T|| (the absolute accuracy of any backward-stable solver): about 11
 // passes of one Sturm sequence per lane where bisection takes 52.
-__global__ void bisect_kernel(const double *dall, const double *eall, const int64_t *eoff, const int *dims,
+// The scaled minors instead of pivots (a division a step): 1577 -> 611 us on a
+// 4x24 m = 2000 density matrix of 31 sectors of up to 857 states.
+__global__ void bisect_kernel(const double *dsall, const double *e2all, const int64_t *eoff, const int *dims,
                               const double *info, const int *esec, int etot, double *evals) {
   const int idx = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (idx >= etot) return;   // uniform in a warp
   const int s = esec[idx], n = dims[s];
   const int k = (int)(idx - eoff[s]);
-  const double *d = dall + eoff[s], *e = eall + eoff[s];
+  const double *ds = dsall + eoff[s], *e2 = e2all + eoff[s];
   const double tnorm = info[4 * s + 2], pivmin = info[4 * s + 3];
   const double pad = 2.0 * EIG_EPS * tnorm + 2.0 * pivmin;
+  const double sc = tridiag_scale(tnorm);
   double lo = info[4 * s + 0] - pad, hi = info[4 * s + 1] + pad;
   for (int it = 0; it < 40; ++it) {
     const double tol = fmax(fmax(2.0 * EIG_EPS * fmax(fabs(lo), fabs(hi)), EIG_EPS * tnorm), pivmin);
     if (hi - lo <= tol) break;
     const double h = (hi - lo) / 33.0;
-    const int c = sturm1(d, e, n, pivmin, lo + (lane + 1) * h);
+    const int c = sturm1(ds, e2, n, (lo + (lane + 1) * h) * sc);
     const unsigned above = __ballot_sync(0xffffffffu, c > k);
     const int f = above ? __ffs(above) - 1 : 32;   // first point above eigenvalue k
     const double nlo = f == 0 ? lo : lo + f * h, nhi = f == 32 ? hi : lo + (f + 1) * h;
@@ -538,23 +624,25 @@ __global__ void inverse_iter_kernel(const double *dall, const double *eall, cons
   double *__restrict__ DL = work + 3 * pl;
   double *__restrict__ X = work + 4 * pl;
 #define AT(arr, i) arr[(size_t)(i) * st + j]
-  // LU = P (T - lam I): row i of U is (U_i, DU_i, DU2_i) at columns i, i+1, i+2
+  // LU = P (T - lam I): row i of U is (1 / U_i, DU_i, DU2_i) at columns i, i+1,
+  // i+2 (the reciprocal once, instead of a division in the chain of every row of
+  // every solve)
   double di = d[0] - lam, dui = n > 1 ? e[0] : 0.0;
   for (int i = 0; i + 1 < n; ++i) {
     const double sub = e[i];
     double dn = d[i + 1] - lam, dun = i + 2 < n ? e[i + 1] : 0.0;
     if (fabs(di) >= fabs(sub) || fabs(sub) < pert) {
-      const double u = fabs(di) < pert ? copysign(pert, di) : di;
-      const double l = sub / u;
-      AT(U, i) = u;
+      const double r = 1.0 / (fabs(di) < pert ? copysign(pert, di) : di);
+      const double l = sub * r;
+      AT(U, i) = r;
       AT(DU, i) = dui;
       AT(DU2, i) = 0.0;
       AT(DL, i) = l;
       piv[(size_t)i * st + j] = 0;
       dn -= l * dui;
     } else {   // rows i and i+1 exchanged
-      const double l = di / sub;
-      AT(U, i) = sub;
+      const double r = 1.0 / sub, l = di * r;
+      AT(U, i) = r;
       AT(DU, i) = dn;
       AT(DU2, i) = dun;
       AT(DL, i) = l;
@@ -565,7 +653,7 @@ __global__ void inverse_iter_kernel(const double *dall, const double *eall, cons
     di = dn;
     dui = dun;
   }
-  AT(U, n - 1) = fabs(di) < pert ? copysign(pert, di) : di;
+  AT(U, n - 1) = 1.0 / (fabs(di) < pert ? copysign(pert, di) : di);
   AT(DU, n - 1) = 0.0;   // read (times zero) by the first back-substitution row
   AT(DU2, n - 1) = 0.0;
   if (n >= 2) AT(DU2, n - 2) = 0.0;
@@ -617,7 +705,7 @@ __global__ void inverse_iter_kernel(const double *dall, const double *eall, cons
     // (the rows loaded but not yet solved are rescaled in registers)
     double x1 = 0.0, x2 = 0.0, mx = 0.0;   // x_{i+1}, x_{i+2}, the largest |x| so far
     auto row = [&](double xv, double du, double du2, double uu, int at, double *ahead, int nahead) {
-      double xi = (xv - du * x1 - du2 * x2) / uu;
+      double xi = (xv - du * x1 - du2 * x2) * uu;
       if (fabs(xi) > 1e250) {
         const double f = 1e-250;
         for (int q = 0; q < n; ++q) AT(X, q) *= f;
@@ -749,7 +837,48 @@ __device__ __forceinline__ double project_off(ZQ zq, int t, const double *h, dou
   return ss;
 }
 
-// One kept block (grp = {sector, first job, count}): classical Gram-Schmidt
+// The vectors of a kept block that inverse iteration left nearly orthogonal,
+// by two matrix products instead of a chain over the vectors.  G = Y^T Y holds
+// every dot product; with E its deviation from I, Gram-Schmidt in descending
+// eigenvalue order (vector j against the vectors q > j) is Y (I - L(E) -
+// diag(E) / 2), L the strictly lower triangle, up to terms of the size of the
+// products of E's columns.  These kernels turn each block's G (grp[b], at
+// goff[b], leading dimension its count) into that factor R for the vectors
+// whose column of E has a norm of at most 1e-8 (so those terms are below
+// 1e-16) and so have all vectors above them; first[b] is the number of
+// vectors this covers, and R leaves the others as they are, for
+// orthonormalize_kernel.  Separated eigenvalues give columns of about
+// eps ||T|| / gap: on a 4x24 m = 2000 density matrix (31 sectors of up to 857
+// states) all blocks are covered, and the stage takes 0.11 ms, 2.77 ms vector
+// by vector.
+// (ortho_check_kernel: a warp per vector; first[b] starts at the count and ends
+// at the index, in descending order, of the first vector not covered.)
+__global__ void __launch_bounds__(256) ortho_check_kernel(const int *grp, const int64_t *goff, const double *Gall,
+                                                          int *first) {
+  const int b = blockIdx.x, cnt = grp[4 * b + 2], lane = threadIdx.x & 31;
+  for (int j = blockIdx.y * 8 + (threadIdx.x >> 5); j < cnt; j += gridDim.y * 8) {
+    const double *g = Gall + goff[b] + (int64_t)j * cnt;
+    double ss = 0.0;
+    for (int q = j + 1 + lane; q < cnt; q += 32) ss += g[q] * g[q];
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const bool fine = ss <= 1e-16 && fabs(g[j] - 1.0) <= 1e-8;   // false for a NaN
+    if (lane == 0 && !fine) atomicMin(first + b, cnt - 1 - j);
+  }
+}
+__global__ void __launch_bounds__(256) ortho_factor_kernel(const int *grp, const int64_t *goff, double *Gall,
+                                                           const int *first) {
+  const int b = blockIdx.x, cnt = grp[4 * b + 2], lane = threadIdx.x & 31, t0 = first[b];
+  for (int j = blockIdx.y * 8 + (threadIdx.x >> 5); j < cnt; j += gridDim.y * 8) {
+    double *g = Gall + goff[b] + (int64_t)j * cnt;
+    const bool in = cnt - 1 - j < t0;
+    const double c = in ? 1.0 - 0.5 * (g[j] - 1.0) : 1.0;   // 1 / the vector's norm
+    __syncwarp();
+    for (int q = lane; q < cnt; q += 32) g[q] = q == j ? c : q > j && in ? -g[q] : 0.0;
+  }
+}
+
+// One kept block (grp = {sector, first job, count}), from vector t_first on
+// (those before it are orthonormal already): classical Gram-Schmidt
 // on its vectors in descending eigenvalue order, so that the dominant states
 // are the least changed; inverse iteration leaves vectors of close
 // eigenvalues only approximately orthogonal (to about eps ||T|| / gap).  The
@@ -772,15 +901,15 @@ __device__ __forceinline__ double project_off(ZQ zq, int t, const double *h, dou
 // good as any basis DSYEV returns for it.  Up to four such vectors are tried.
 // status bit 1: a vector stayed dependent (or its cluster is not at the
 // bottom of the spectrum).
-__device__ void ortho_one(int blk, const int *grp, const int *dims, const int64_t *eoff, const double *evals,
-                          const double *info, const int *job_k, double *Y, int ldy, int *status, double *h,
-                          double *red) {
+__device__ void ortho_one(int blk, int t_first, const int *grp, const int *dims, const int64_t *eoff,
+                          const double *evals, const double *info, const int *job_k, double *Y, int ldy, int *status,
+                          double *h, double *red) {
   const int s = grp[4 * blk], j0 = grp[4 * blk + 1], cnt = grp[4 * blk + 2];
   const int n = dims[s], tid = threadIdx.x;
   const double lam_min = evals[eoff[s]], cluster = 1e4 * EIG_EPS * info[4 * s + 2];
   double *gp = h + cnt;   // project_off's group parts
   auto vec = [&](int q) -> const double * { return Y + (size_t)(j0 + cnt - 1 - q) * ldy; };
-  for (int t = 1; t < cnt; ++t) {
+  for (int t = t_first; t < cnt; ++t) {
     const int jt = j0 + cnt - 1 - t;
     double *y = Y + (size_t)jt * ldy;
     bool ok = false;
@@ -831,7 +960,7 @@ __device__ void ortho_one(int blk, const int *grp, const int *dims, const int64_
 // every CTA has passed the barrier that follows its reads.  A CTA reads and
 // writes only its own rows of the vectors in global memory.
 template <int CL>
-__device__ void ortho_coop(cg::cluster_group &cl, int rank, int blk, const int *grp, const int *dims,
+__device__ void ortho_coop(cg::cluster_group &cl, int rank, int blk, int t_first, const int *grp, const int *dims,
                            const int64_t *eoff, const double *evals, const double *info, const int *job_k, double *Y,
                            int ldy, int *status, double *sm, double *red) {
   const int s = grp[4 * blk], j0 = grp[4 * blk + 1], cnt = grp[4 * blk + 2];
@@ -854,7 +983,7 @@ __device__ void ortho_coop(cg::cluster_group &cl, int rank, int blk, const int *
     return tot;
   };
   auto vec = [&](int q) { return Y + (size_t)(j0 + cnt - 1 - q) * ldy; };   // q-th vector in descending order
-  for (int t = 1; t < cnt; ++t) {
+  for (int t = t_first; t < cnt; ++t) {
     double *y = vec(t);
     const int jt = j0 + cnt - 1 - t;
     bool ok = false;
@@ -919,17 +1048,17 @@ __device__ void ortho_coop(cg::cluster_group &cl, int rank, int blk, const int *
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(ORTH_THREADS, 1)
     orthonormalize_kernel(const int *oblk, const int *obig, const int *grp, const int *dims, const int64_t *eoff,
-                          const double *evals, const double *info, const int *job_k, double *Y, int ldy,
-                          int *status) {
+                          const double *evals, const double *info, const int *job_k, const int *first, double *Y,
+                          int ldy, int *status) {
   extern __shared__ double sm[];
   __shared__ double red[64];
   cg::cluster_group cl = cg::this_cluster();
   const int b = blockIdx.x / CL, rank = (int)cl.block_rank();
   const int blk = oblk[blockIdx.x];
   if (obig[b])
-    ortho_coop<CL>(cl, rank, blk, grp, dims, eoff, evals, info, job_k, Y, ldy, status, sm, red);
+    ortho_coop<CL>(cl, rank, blk, max(first[blk], 1), grp, dims, eoff, evals, info, job_k, Y, ldy, status, sm, red);
   else if (blk >= 0)
-    ortho_one(blk, grp, dims, eoff, evals, info, job_k, Y, ldy, status, sm, red);
+    ortho_one(blk, max(first[blk], 1), grp, dims, eoff, evals, info, job_k, Y, ldy, status, sm, red);
 }
 
 // Back-transformation of the kept vectors, one warp per vector and the
@@ -982,104 +1111,248 @@ __global__ void backtransform_kernel(const double *Aall, const int64_t *off, con
   for (int i = lane; i < n; i += 32) dst[i] = sg * col[i];
 }
 
-// The same back-transformation with each warp's vector in registers (lane l
-// holds rows l + 32 r, r < RPL) for sectors of up to 32 RPL states: the CTA's
-// BT_WARPS warps (vectors of one kept block, so of one sector) share the
-// reflectors, staged kb at a time in shared memory by one coalesced load of
-// the whole CTA, so that a step waits for no L2 load.  A lane's rows stay
-// fixed (backtransform_kernel's shift with k), so the dot products are
-// grouped differently: the two agree to rounding.  Warps past the block's
-// last vector take part in the loads and barriers only.
-constexpr int BT_WARPS = 8;
-template <int RPL>
-__global__ void __launch_bounds__(32 * BT_WARPS)
-    backtransform_reg_kernel(const double *Aall, const int64_t *off, const double *tauall, const int64_t *eoff,
-                             const int *dims, const int *grp, const int *slab, const double *Y, int ldy,
-                             const int64_t *job_dst, double *out, int kb) {
-  extern __shared__ double sv[];   // kb reflectors of n rows
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = blockDim.x;
-  const int g = slab[2 * blockIdx.x], c = slab[2 * blockIdx.x + 1] + warp;
-  const int s = grp[4 * g], j0 = grp[4 * g + 1], cnt = grp[4 * g + 2];
-  const bool active = c < cnt;
-  const int n = dims[s], j = j0 + c;
+// The same back-transformation by matrix products, for sectors of up to
+// 1536 states (a CTA's shared memory): BT_NB consecutive reflectors are one block reflector I - V T V^T
+// (T upper triangular, by wy_t_kernel), applied to a CTA's 8 VT vectors of one
+// kept block.  Vector by vector, each reflector is a dot product over the
+// vector, a reduction across the warp and an update: a chain of some 300
+// cycles for each of the sector's states (1.8 ms on the 4x24 m = 2000 density
+// matrix with 857 states).  A block reflector has three barriers, and its
+// products run on DMMA: 0.24 ms, and 0.05 ms for the T of all blocks.
+//
+// The vectors stay in registers as Y^T in accumulator layout: warp w holds the
+// row tiles (8 rows) w, w + BT_WARPS, ..., lane (g, t) of tile j the entries
+// (vector g, rows 2t and 2t + 1).  As the left operand of Y^T V an accumulator
+// register is a fragment as it stands when the inner dimension is taken in the
+// order rows 0, 2, 4, 6, then 1, 3, 5, 7; V is read to match.  Each warp keeps
+// its own rows of the block's reflectors in shared memory, a tile's entry
+// (row r, reflector q) at 8 q + (r with bit 2 flipped where q has bit 1).
+constexpr int BT_WARPS = 16, BT_NB = 16;
+
+// T of the block reflectors (LAPACK dlarft, forward and columnwise): block b of
+// the grid makes T of reflectors [16 p, 16 p + 16) of sector s, pan[2b] = s,
+// pan[2b + 1] = p, from the dot products of the reflectors.  Column-major.
+__global__ void __launch_bounds__(256) wy_t_kernel(const double *Aall, const int64_t *off, const double *tauall,
+                                                   const int64_t *eoff, const int *dims, const int *pan, double *Tall) {
+  __shared__ double vs[BT_NB][65], G[BT_NB][BT_NB + 1], T[BT_NB][BT_NB + 1];
+  const int s = pan[2 * blockIdx.x], k0 = pan[2 * blockIdx.x + 1] * BT_NB, n = dims[s], tid = threadIdx.x;
   const double *A = Aall + off[s], *tau = tauall + eoff[s];
-  double col[RPL];
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int i = lane + 32 * r;
-    col[r] = active && i < n ? Y[(size_t)j * ldy + i] : 0.0;
-  }
-  for (int k0 = n - 2; k0 >= 0; k0 -= kb) {
-    const int nk = min(kb, k0 + 1);   // reflectors k0, k0 - 1, ..., k0 - nk + 1
-    __syncthreads();                  // the previous chunk is read
-    for (int u = 0; u < nk; ++u) {
-      const int k = k0 - u;
-      const double *v = A + (int64_t)k * n;
-      for (int i = k + 1 + (int)threadIdx.x; i < n; i += nt) sv[(size_t)u * n + i] = v[i];
+  const int i = tid >> 4, j = tid & 15;
+  double acc = 0.0;
+  for (int r0 = (k0 + 1) & ~63; r0 < n; r0 += 64) {
+    __syncthreads();
+    for (int e = tid; e < BT_NB * 64; e += 256) {
+      const int q = e >> 6, r = r0 + (e & 63), k = k0 + q;
+      vs[q][e & 63] = k + 1 < n && r > k && r < n ? A[(int64_t)k * n + r] : 0.0;
     }
     __syncthreads();
-    if (!active) continue;
-    for (int u = 0; u < nk; ++u) {
-      const int k = k0 - u;
-      const double t = tau[k];
-      if (t == 0.0) continue;
-      const double *v = sv + (size_t)u * n;
-      // rows 32 r .. 32 r + 31 all at or above k are skipped by the whole
-      // warp; two partial sums (even and odd r) shorten the chain of adds
-      double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 8
+    for (int r = 0; r < 64; ++r) acc += vs[i][r] * vs[j][r];
+  }
+  G[i][j] = acc;
+  T[i][j] = 0.0;
+  __syncthreads();
+  for (int c = 0; c < BT_NB; ++c) {
+    const double t = k0 + c + 1 < n ? tau[k0 + c] : 0.0;
+    if (tid < c) {
+      double x = 0.0;
+      for (int q = tid; q < c; ++q) x += T[tid][q] * G[q][c];
+      T[tid][c] = -t * x;
+    }
+    if (tid == c) T[c][c] = t;
+    __syncthreads();
+  }
+  Tall[(int64_t)blockIdx.x * (BT_NB * BT_NB) + j * BT_NB + i] = T[i][j];
+}
+
+__device__ __forceinline__ void bt_dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// shared memory of a CTA: the reflectors of a block, the warps' parts of Y^T V
+// (later the largest entries), Y^T V, its product with T^T, and T
+constexpr int bt_smem_doubles(int tiles, int vt) {
+  return BT_WARPS * (tiles * 8 * BT_NB + 8 * vt * BT_NB) + 2 * 8 * vt * BT_NB + BT_NB * BT_NB;
+}
+
+// TILES: row tiles of a warp; pan0[s]: index of sector s's first T.
+template <int TILES, int VT>
+__global__ void __launch_bounds__(32 * BT_WARPS, 1)
+    backtransform_wy_kernel(const double *Aall, const int64_t *off, const double *Tall, const int *pan0, const int *dims,
+                            const int *grp, const int *slab, const double *Y, int ldy, const int64_t *job_dst,
+                            double *out) {
+  extern __shared__ double bsm[];
+  constexpr int NV = 8 * VT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  double *vw = bsm + warp * (TILES * 8 * BT_NB);
+  double *parts = bsm + BT_WARPS * TILES * 8 * BT_NB, *S = parts + BT_WARPS * NV * BT_NB, *Zt = S + NV * BT_NB,
+         *T = Zt + NV * BT_NB;
+  const int gi = slab[2 * blockIdx.x], c0 = slab[2 * blockIdx.x + 1];
+  const int s = grp[4 * gi], j0 = grp[4 * gi + 1], cnt = grp[4 * gi + 2], n = dims[s];
+  const double *A = Aall + off[s];
+  double y[TILES][VT][2];
 #pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (32 * r + 31 > k && i > k && i < n) {
-          if (r & 1)
-            acc1 += v[i] * col[r];
-          else
-            acc0 += v[i] * col[r];
+  for (int j = 0; j < TILES; ++j)
+#pragma unroll
+    for (int v = 0; v < VT; ++v)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * v + g, r = 8 * (warp + BT_WARPS * j) + 2 * t + e;
+        y[j][v][e] = c < cnt && r < n ? Y[(int64_t)(j0 + c) * ldy + r] : 0.0;
+      }
+  const int np = (n - 1 + BT_NB - 1) / BT_NB;   // blocks of the n - 1 reflectors
+  for (int p = np - 1; p >= 0; --p) {
+    const int k0 = p * BT_NB;
+    // the warp's rows of the reflectors: zero up to their own index; row tiles
+    // that end above the block's first row are zero throughout
+#pragma unroll
+    for (int j = 0; j < TILES; ++j) {
+      const int r0 = 8 * (warp + BT_WARPS * j), r = r0 + (lane & 7);
+      if (r0 + 7 <= k0 || r0 >= n) continue;
+#pragma unroll
+      for (int u = 0; u < BT_NB / 4; ++u) {
+        const int q = (lane >> 3) + 4 * u, k = k0 + q;
+        vw[j * 8 * BT_NB + q * 8 + ((lane & 7) ^ ((q & 2) << 1))] =
+            k + 1 < n && r > k && r < n ? A[(int64_t)k * n + r] : 0.0;
+      }
+    }
+    if (tid < BT_NB * BT_NB) T[tid] = Tall[(int64_t)(pan0[s] + p) * (BT_NB * BT_NB) + tid];
+    __syncwarp();
+    // Y^T V of the warp's rows
+    double w[VT][BT_NB / 8][2];
+#pragma unroll
+    for (int v = 0; v < VT; ++v)
+#pragma unroll
+      for (int h = 0; h < BT_NB / 8; ++h) w[v][h][0] = w[v][h][1] = 0.0;
+#pragma unroll
+    for (int j = 0; j < TILES; ++j) {
+      const int r0 = 8 * (warp + BT_WARPS * j);
+      if (r0 + 7 <= k0 || r0 >= n) continue;
+#pragma unroll
+      for (int h = 0; h < BT_NB / 8; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int q = 8 * h + g;
+          const double b = vw[j * 8 * BT_NB + q * 8 + ((2 * t + e) ^ ((q & 2) << 1))];
+#pragma unroll
+          for (int v = 0; v < VT; ++v) bt_dmma(w[v][h], y[j][v][e], b);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < VT; ++v)
+#pragma unroll
+      for (int h = 0; h < BT_NB / 8; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) parts[warp * (NV * BT_NB) + (8 * v + g) * BT_NB + 8 * h + 2 * t + e] = w[v][h][e];
+    __syncthreads();
+    if (tid < NV * BT_NB) {
+      double x = 0.0;
+#pragma unroll
+      for (int q = 0; q < BT_WARPS; ++q) x += parts[q * (NV * BT_NB) + tid];
+      S[tid] = x;
+    }
+    __syncthreads();
+    if (tid < NV * BT_NB) {   // (Y^T V T^T)[vector][q] = sum_i T[q][i] S[vector][i]
+      const int v = tid / BT_NB, q = tid % BT_NB;
+      double x = 0.0;
+#pragma unroll
+      for (int i = 0; i < BT_NB; ++i) x += T[i * BT_NB + q] * S[v * BT_NB + i];
+      Zt[tid] = -x;
+    }
+    __syncthreads();
+    // Y^T -= (Y^T V T^T) V^T
+    double a[VT][BT_NB / 4];
+#pragma unroll
+    for (int v = 0; v < VT; ++v)
+#pragma unroll
+      for (int kk = 0; kk < BT_NB / 4; ++kk) a[v][kk] = Zt[(8 * v + g) * BT_NB + 4 * kk + t];
+#pragma unroll
+    for (int j = 0; j < TILES; ++j) {
+      const int r0 = 8 * (warp + BT_WARPS * j);
+      if (r0 + 7 <= k0 || r0 >= n) continue;
+#pragma unroll
+      for (int kk = 0; kk < BT_NB / 4; ++kk) {
+        const int q = 4 * kk + t;
+        const double b = vw[j * 8 * BT_NB + q * 8 + (g ^ ((q & 2) << 1))];
+#pragma unroll
+        for (int v = 0; v < VT; ++v) bt_dmma(y[j][v], a[v][kk], b);
+      }
+    }
+    __syncwarp();   // the warp's reflectors are read
+  }
+  // the sign of each vector's entry of largest magnitude (the first of equal
+  // ones), over the lane's rows, the four lanes of a vector, the warps
+  __shared__ int bidx[BT_WARPS][NV];
+#pragma unroll
+  for (int v = 0; v < VT; ++v) {
+    double best = 0.0;   // the entry itself
+    int bi = 1 << 30;
+#pragma unroll
+    for (int j = 0; j < TILES; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = 8 * (warp + BT_WARPS * j) + 2 * t + e;
+        if (r < n && (fabs(y[j][v][e]) > fabs(best) || bi == 1 << 30)) {
+          best = y[j][v][e];
+          bi = r;
         }
       }
-      double acc = acc0 + acc1;
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      const double f = t * acc;
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (32 * r + 31 > k && i > k && i < n) col[r] -= f * v[i];
+    for (int o = 1; o < 4; o <<= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (fabs(ob) > fabs(best) || (fabs(ob) == fabs(best) && oi < bi)) {
+        best = ob;
+        bi = oi;
       }
     }
-  }
-  if (!active) return;
-  double best = -1.0;
-  int bi = 0;
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int i = lane + 32 * r;
-    if (i < n && fabs(col[r]) > best) {
-      best = fabs(col[r]);
-      bi = i;
+    if (t == 0) {
+      parts[warp * NV + 8 * v + g] = best;
+      bidx[warp][8 * v + g] = bi;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ob > best || (ob == best && oi < bi)) {
-      best = ob;
-      bi = oi;
+  __syncthreads();
+  if (tid < NV) {
+    double best = parts[tid];
+    int bi = bidx[0][tid];
+    for (int q = 1; q < BT_WARPS; ++q) {
+      const double ob = parts[q * NV + tid];
+      const int oi = bidx[q][tid];
+      if (fabs(ob) > fabs(best) || (fabs(ob) == fabs(best) && oi < bi)) {
+        best = ob;
+        bi = oi;
+      }
+    }
+    S[tid] = best < 0.0 ? -1.0 : 1.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < VT; ++v) {
+    const int c = c0 + 8 * v + g;
+    if (c < cnt) {
+      const double sg = S[8 * v + g];
+      double *dst = out + job_dst[j0 + c];
+#pragma unroll
+      for (int j = 0; j < TILES; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int r = 8 * (warp + BT_WARPS * j) + 2 * t + e;
+          if (r < n) dst[r] = sg * y[j][v][e];
+        }
     }
   }
-  // the sign of the entry of largest magnitude: the lane holding row bi
-  // broadcasts it
-  double atbi = 0.0;
-#pragma unroll
-  for (int r = 0; r < RPL; ++r)
-    if (lane + 32 * r == bi) atbi = col[r];
-  atbi = __shfl_sync(0xffffffffu, atbi, bi & 31);
-  const double sg = atbi < 0.0 ? -1.0 : 1.0;
-  double *dst = out + job_dst[j];
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int i = lane + 32 * r;
-    if (i < n) dst[i] = sg * col[r];
-  }
+}
+
+// |psi|^2 from its block sums, and 1 / |psi|^2 as the coefficient of every task
+// of the density matrix
+__global__ void rho_scale_kernel(const double *part, int npart, Task *tasks, int ntasks, double *nrm2) {
+  __shared__ double red[32];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < npart; i += blockDim.x) s += part[i];
+  s = block_sum(s, red);
+  for (int i = threadIdx.x; i < ntasks; i += blockDim.x) tasks[i].coef = 1.0 / s;
+  if (threadIdx.x == 0) *nrm2 = s;
 }
 
 }  // namespace tjb
@@ -1128,6 +1401,31 @@ uint64_t hash_data(const double *p, int64_t n) {
 }
 
 size_t al256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Host tables gathered into one buffer for one copy to the device, each at a
+// 256-byte border; room() is device space behind them that nothing is copied
+// into (so it comes last).
+struct Tables {
+  std::vector<char> buf;
+  size_t extra = 0;
+  size_t zeros(size_t bytes) {
+    const size_t at = buf.size();
+    buf.resize(at + al256(std::max<size_t>(bytes, 1)), 0);
+    return at;
+  }
+  template <class T>
+  size_t add(const std::vector<T> &v) {
+    const size_t at = zeros(v.size() * sizeof(T));
+    if (!v.empty()) std::memcpy(buf.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+  size_t room(size_t bytes) {
+    const size_t at = size();
+    extra += al256(std::max<size_t>(bytes, 1));
+    return at;
+  }
+  size_t size() const { return buf.size() + extra; }
+};
 
 // Clusters of 16 CTAs (a non-portable size) where the GPU can schedule one
 // with `threads` threads and `smem` bytes of dynamic shared memory per CTA;
@@ -1191,18 +1489,11 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     tc.dev = nullptr;
     tc.len = 0;
     CKT(cudaEventRecord(ctx->tev[0], st));
-    // psi on the device and its norm
+    // psi on the device
     int rc;
     if ((rc = ctx->trA.reserve(sizeof(double) * (D + 4)))) return rc;
     double *psi = ctx->trA.d();
     CKT(upload(ctx, psi, wave->data, D, st));
-    double acc[4] = {0, 0, 0, 0};   // four independent sums, added at the end
-    int64_t i = 0;
-    for (; i + 4 <= D; i += 4)
-      for (int q = 0; q < 4; ++q) acc[q] += wave->data[i + q] * wave->data[i + q];
-    for (; i < D; ++i) acc[0] += wave->data[i] * wave->data[i];
-    const double nrm2 = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-    if (!(nrm2 > 0) || !std::isfinite(nrm2)) return set_err(TJ_ERR_NUMERIC, "tj_truncation: zero or non-finite psi");
     // rho per sector as one grouped-GEMM pass
     std::vector<Cell> cells;
     std::vector<Task> tasks;
@@ -1235,35 +1526,28 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       t.L.trans = (int8_t)(side == 0 ? 0 : 1);
       t.R = t.L;
       t.R.trans = (int8_t)(side == 0 ? 1 : 0);
-      t.coef = 1.0 / nrm2;
+      t.coef = 1.0;   // rho_scale_kernel sets 1 / |psi|^2
       t.K = K;
       if (n > 0 && K > 0) tasks.push_back(t);
       c.t_end = (int)tasks.size();
-      const int ci = (int)cells.size();
       cells.push_back(c);
-      for (int r0 = 0; r0 < n; r0 += BM)
-        for (int c0 = 0; c0 < n; c0 += BN) tiles.push_back(Tile{ci, r0, c0, c.t_begin, c.t_end, c.t_end, c.t_end, -1});
     }
+    // work items in order of weight (one sector of 857 states holds a fifth of
+    // a density matrix's products)
+    std::vector<Reduce> red;
+    int64_t nslots = 0;
+    split_tiles(cells, tasks, tiles, red, nslots, false);
     const int maxn = std::max(1, *std::max_element(dims.begin(), dims.end()));
     // sectors largest first for the one-CTA-per-sector reduction
     std::vector<int> order(nsec);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return dims[a] > dims[b]; });
-    // trD: d, e, tau, eigenvalues (etot each), then 4 per sector
+    // trD: d, e, tau, eigenvalues, scaled d, scaled e^2 (etot each), then 4 per sector
     if ((rc = ctx->trB.reserve(sizeof(double) * (rlen + 4))) ||
-        (rc = ctx->trD.reserve(sizeof(double) * (4 * etot + 4 * nsec + 8))))
+        (rc = ctx->trD.reserve(sizeof(double) * (6 * etot + 4 * nsec + 8))))
       return rc;
-    double *dd = ctx->trD.d(), *de = dd + etot, *dtau = de + etot, *dev = dtau + etot, *dinfo = dev + etot;
-    // small tables packed into one buffer
-    const size_t tb = cells.size() * sizeof(Cell), kb = tasks.size() * sizeof(Task), lb = tiles.size() * sizeof(Tile);
-    const size_t ob = nsec * sizeof(int64_t), db = nsec * sizeof(int);
-    size_t pos = 0;
-    const size_t p_cells = pos; pos += al256(tb);
-    const size_t p_tasks = pos; pos += al256(kb);
-    const size_t p_tiles = pos; pos += al256(lb);
-    const size_t p_roff = pos; pos += al256(ob);
-    const size_t p_eoff = pos; pos += al256(ob);
-    const size_t p_dims = pos; pos += al256(db);
+    double *dd = ctx->trD.d(), *de = dd + etot, *dtau = de + etot, *dev = dtau + etot, *dds = dev + etot,
+           *de2 = dds + etot, *dinfo = de2 + etot;
     // clusters of the tridiagonal reduction: one per large sector, then the
     // small sectors tcl at a time (largest first)
     // shared memory: the per-sector vectors, and for a sector reduced by a
@@ -1294,24 +1578,16 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       }
     }
     const int nclus = (int)tbig.size();
-    const size_t p_tsec = pos; pos += al256(sizeof(int) * std::max<size_t>(tsec.size(), 1));
-    const size_t p_tbig = pos; pos += al256(sizeof(int) * std::max<size_t>(tbig.size(), 1));
-    const size_t p_esec = pos; pos += al256(sizeof(int) * (size_t)std::max<int64_t>(etot, 1));
-    const size_t p_cnt = pos; pos += 256;
-    if ((rc = ctx->trE.reserve(pos))) return rc;
+    // the small tables in one buffer and one copy
+    Tables tab;
+    const size_t p_cells = tab.add(cells), p_tasks = tab.add(tasks), p_tiles = tab.add(tiles), p_red = tab.add(red);
+    const size_t p_roff = tab.add(roff), p_eoff = tab.add(eoff), p_dims = tab.add(dims), p_tsec = tab.add(tsec);
+    const size_t p_tbig = tab.add(tbig), p_esec = tab.add(esec), p_cnt = tab.zeros(256);
+    const int ndot = dot_blocks(D);
+    const size_t p_part = tab.room(sizeof(double) * (ndot + 1));   // partial sums of |psi|^2, then |psi|^2
+    if ((rc = ctx->trE.reserve(tab.size())) || (rc = ctx->trC.reserve(sizeof(double) * (nslots * BM * BN + 4)))) return rc;
     char *tbase = (char *)ctx->trE.p;
-    CKT(cudaMemcpyAsync(tbase + p_cells, cells.data(), tb, cudaMemcpyHostToDevice, st));
-    if (kb) CKT(cudaMemcpyAsync(tbase + p_tasks, tasks.data(), kb, cudaMemcpyHostToDevice, st));
-    CKT(cudaMemcpyAsync(tbase + p_tiles, tiles.data(), lb, cudaMemcpyHostToDevice, st));
-    CKT(cudaMemcpyAsync(tbase + p_roff, roff.data(), ob, cudaMemcpyHostToDevice, st));
-    CKT(cudaMemcpyAsync(tbase + p_eoff, eoff.data(), ob, cudaMemcpyHostToDevice, st));
-    CKT(cudaMemcpyAsync(tbase + p_dims, dims.data(), db, cudaMemcpyHostToDevice, st));
-    if (nclus) {
-      CKT(cudaMemcpyAsync(tbase + p_tsec, tsec.data(), sizeof(int) * tsec.size(), cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(tbase + p_tbig, tbig.data(), sizeof(int) * tbig.size(), cudaMemcpyHostToDevice, st));
-    }
-    if (etot) CKT(cudaMemcpyAsync(tbase + p_esec, esec.data(), sizeof(int) * etot, cudaMemcpyHostToDevice, st));
-    CKT(cudaMemsetAsync(tbase + p_cnt, 0, 256, st));
+    CKT(cudaMemcpyAsync(tbase, tab.buf.data(), tab.buf.size(), cudaMemcpyHostToDevice, st));
     const int64_t *d_roff = (const int64_t *)(tbase + p_roff), *d_eoff = (const int64_t *)(tbase + p_eoff);
     const int *d_dims = (const int *)(tbase + p_dims);
     int *d_status = (int *)(tbase + p_cnt + 16);
@@ -1325,7 +1601,12 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     g.tiles = (const Tile *)(tbase + p_tiles);
     g.ntiles = (int)tiles.size();
     g.counter = (unsigned int *)(tbase + p_cnt);
+    g.slots = ctx->trC.d();
+    double *part = (double *)(tbase + p_part);
+    launch_dot(psi, psi, D, part, ndot, st);
+    rho_scale_kernel<<<1, 256, 0, st>>>(part, ndot, (Task *)(tbase + p_tasks), (int)tasks.size(), part + ndot);
     launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
+    launch_reduce(g, (const Reduce *)(tbase + p_red), (int)red.size(), st);
     CKT(cudaGetLastError());
     CKT(cudaEventRecord(ctx->tev[1], st));
     // tridiagonal reduction, then all eigenvalues
@@ -1334,24 +1615,27 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       if (tcl == 16) {
         CKT(cudaFuncSetAttribute(tridiag_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<16><<<nclus * 16, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
-                                                                 dd, de, dtau, dinfo, (int64_t)(tsm / 8));
+                                                                 dd, de, dtau, dinfo, dds, de2, (int64_t)(tsm / 8));
       } else {
         CKT(cudaFuncSetAttribute(tridiag_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<8><<<nclus * 8, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
-                                                               dd, de, dtau, dinfo, (int64_t)(tsm / 8));
+                                                               dd, de, dtau, dinfo, dds, de2, (int64_t)(tsm / 8));
       }
       CKT(cudaGetLastError());
     }
     CKT(cudaEventRecord(ctx->tev[2], st));
     if (etot) {
-      bisect_kernel<<<(unsigned)((etot + 3) / 4), 128, 0, st>>>(dd, de, d_eoff, d_dims, dinfo,
+      bisect_kernel<<<(unsigned)((etot + 3) / 4), 128, 0, st>>>(dds, de2, d_eoff, d_dims, dinfo,
                                                                     (const int *)(tbase + p_esec), (int)etot, dev);
       CKT(cudaGetLastError());
     }
     std::vector<double> ev(etot);
+    CKT(cudaMemcpyAsync(ctx->pinned, part + ndot, sizeof(double), cudaMemcpyDeviceToHost, st));
     CKT(cudaMemcpyAsync(ev.data(), dev, sizeof(double) * etot, cudaMemcpyDeviceToHost, st));
     CKT(cudaEventRecord(ctx->tev[3], st));
     CKT(cudaStreamSynchronize(st));
+    const double nrm2 = ctx->pinned[0];
+    if (!(nrm2 > 0) || !std::isfinite(nrm2)) return set_err(TJ_ERR_NUMERIC, "tj_truncation: zero or non-finite psi");
     const auto sel0 = std::chrono::steady_clock::now();
     float stage_ms[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int i = 0; i < 3; ++i) CKT(cudaEventElapsedTime(&stage_ms[i], ctx->tev[i], ctx->tev[i + 1]));
@@ -1449,24 +1733,86 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     tc.len = dpos;
     const int njobs = (int)job_sec.size(), ngrp = (int)grp.size() / 4;
     if (njobs > 0) {
-      // back-transformation: vectors in registers (BT_WARPS to a CTA) for
-      // sectors of up to 32 * 48 states, else in shared memory (W warps)
-      const bool bt_reg = maxn <= 32 * 48;
-      const int W = bt_reg ? BT_WARPS : std::max(1, std::min(32, (int)(196608 / (sizeof(double) * maxn))));
+      // back-transformation: blocks of reflectors on 16 vectors (8 for sectors
+      // above 1024 states, whose rows would not fit the registers) a CTA, else
+      // (above 1536) vector by vector in shared memory, W warps
+      const bool bt_wy = maxn <= 1536;
+      const int W = bt_wy ? (maxn <= 1024 ? 16 : 8) : std::max(1, std::min(32, (int)(196608 / (sizeof(double) * maxn))));
+      std::vector<int> pan, pan0(nsec, 0);
+      if (bt_wy)
+        for (int b = 0; b < ngrp; ++b) {
+          const int x = grp[4 * b];
+          pan0[x] = (int)pan.size() / 2;
+          for (int q = 0; q * BT_NB < dims[x] - 1; ++q) pan.insert(pan.end(), {x, q});
+        }
+      const int npan = (int)pan.size() / 2;
       for (int b = 0; b < ngrp; ++b)
         for (int c0 = 0; c0 < grp[4 * b + 2]; c0 += W) slab.insert(slab.end(), {b, c0});
       const int nslab = (int)slab.size() / 2;
       const int ldy = (maxn + 3) / 4 * 4;
-      // trC: inverse-iteration factors and vectors; trA: job tables and the operator
+      // trC: inverse-iteration factors and vectors; trA: tables and the operator
       const size_t wpl = (size_t)maxn * njobs;
       const size_t p_work = 0, p_y = p_work + al256(5 * wpl * 8), p_piv = p_y + al256((size_t)njobs * ldy * 8);
-      if ((rc = ctx->trC.reserve(p_piv + al256(wpl)))) return rc;
-      size_t q = 0;
-      const size_t q_sec = q; q += al256((size_t)njobs * 4);
-      const size_t q_k = q; q += al256((size_t)njobs * 4);
-      const size_t q_dst = q; q += al256((size_t)njobs * 8);
-      const size_t q_grp = q; q += al256(grp.size() * 4);
-      const size_t q_slab = q; q += al256(slab.size() * 4);
+      // the two products of the orthonormalisation: G = Y^T Y of every block
+      // (its lower triangle of tiles), and Z = Y R by column tiles, R lower
+      // triangular
+      std::vector<Cell> ocells;
+      std::vector<Task> otasks;
+      std::vector<Tile> gtiles, ztiles;
+      std::vector<int64_t> goff(ngrp);
+      int64_t glen = 0;
+      {
+        auto opnd = [&](int64_t off, int ld, int8_t space, int8_t trans) {
+          Operand o;
+          std::memset(&o, 0, sizeof o);
+          o.off = off;
+          o.ld = ld;
+          o.space = space;
+          o.trans = trans;
+          return o;
+        };
+        auto cell = [&](int64_t off, int ld, int M, int N, const Operand &L, const Operand &R, int K) {
+          Cell c;
+          std::memset(&c, 0, sizeof c);
+          c.off = off;
+          c.ld = ld;
+          c.M = M;
+          c.N = N;
+          c.t_begin = (int)otasks.size();
+          Task t;
+          std::memset(&t, 0, sizeof t);
+          t.L = L;
+          t.R = R;
+          t.coef = 1.0;
+          t.K = K;
+          otasks.push_back(t);
+          c.t_end = (int)otasks.size();
+          ocells.push_back(c);
+        };
+        auto tile = [&](std::vector<Tile> &v, int r0, int c0) {
+          const int ci = (int)ocells.size() - 1, t = ocells[ci].t_begin;
+          v.push_back(Tile{ci, r0, c0, t, t + 1, t + 1, t + 1, -1});
+        };
+        for (int b = 0; b < ngrp; ++b) {
+          const int n = dims[grp[4 * b]], cnt = grp[4 * b + 2];
+          const int64_t y0 = (int64_t)grp[4 * b + 1] * ldy;
+          goff[b] = glen;
+          glen += ((int64_t)cnt * cnt + 3) / 4 * 4;
+          cell(goff[b], cnt, cnt, cnt, opnd(y0, ldy, SP_PSI, 1), opnd(y0, ldy, SP_PSI, 0), n);
+          for (int c0 = 0; c0 < cnt; c0 += BN)
+            for (int r0 = c0 / BM * BM; r0 < cnt; r0 += BM) tile(gtiles, r0, c0);
+          for (int c0 = 0; c0 < cnt; c0 += BN) {
+            cell(y0 + (int64_t)c0 * ldy, ldy, n, std::min(BN, cnt - c0), opnd(y0 + (int64_t)c0 * ldy, ldy, SP_PSI, 0),
+                 opnd(goff[b] + (int64_t)c0 * cnt + c0, cnt, SP_SCR, 0), cnt - c0);
+            for (int r0 = 0; r0 < n; r0 += BM) tile(ztiles, r0, 0);
+          }
+        }
+        // longest inner dimension first
+        for (auto *v : {&gtiles, &ztiles})
+          std::stable_sort(v->begin(), v->end(), [&](const Tile &a, const Tile &b) { return otasks[a.tb].K > otasks[b.tb].K; });
+      }
+      const size_t p_z = p_piv + al256(wpl), p_g = p_z + al256((size_t)njobs * ldy * 8);
+      if ((rc = ctx->trC.reserve(p_g + al256((size_t)glen * 8)))) return rc;
       // clusters of the orthonormalisation: one per large kept block (cnt^2 n
       // above 3e7), then the other blocks ocl at a time, largest first
       const size_t osm = sizeof(double) * (3 * (size_t)maxn + (maxn + 7) / 8 + 8 + ORTH_THREADS);
@@ -1488,19 +1834,19 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
         }
       }
       const int nocl = (int)obig.size();
-      const size_t q_oblk = q; q += al256(oblk.size() * 4);
-      const size_t q_obig = q; q += al256(obig.size() * 4);
-      const size_t q_out = q; q += al256((size_t)dpos * 8);
-      if ((rc = ctx->trA.reserve(q))) return rc;   // psi is no longer needed
+      Tables tab2;
+      const size_t q_sec = tab2.add(job_sec), q_k = tab2.add(job_k), q_dst = tab2.add(job_dst), q_grp = tab2.add(grp);
+      const size_t q_slab = tab2.add(slab), q_oblk = tab2.add(oblk), q_obig = tab2.add(obig), q_cells = tab2.add(ocells);
+      const size_t q_tasks = tab2.add(otasks), q_gt = tab2.add(gtiles), q_zt = tab2.add(ztiles), q_goff = tab2.add(goff);
+      const size_t q_pan = tab2.add(pan), q_pan0 = tab2.add(pan0);
+      std::vector<int> first(ngrp);
+      for (int b = 0; b < ngrp; ++b) first[b] = grp[4 * b + 2];
+      const size_t q_cnt = tab2.zeros(256), q_first = tab2.add(first);
+      const size_t q_wyt = tab2.room(sizeof(double) * BT_NB * BT_NB * npan), q_out = tab2.room((size_t)dpos * 8);
+      if ((rc = ctx->trA.reserve(tab2.size()))) return rc;   // psi is no longer needed
       char *ab = (char *)ctx->trA.p, *cb = (char *)ctx->trC.p;
-      CKT(cudaMemcpyAsync(ab + q_sec, job_sec.data(), (size_t)njobs * 4, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_k, job_k.data(), (size_t)njobs * 4, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_dst, job_dst.data(), (size_t)njobs * 8, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_grp, grp.data(), grp.size() * 4, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_slab, slab.data(), slab.size() * 4, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_oblk, oblk.data(), oblk.size() * 4, cudaMemcpyHostToDevice, st));
-      CKT(cudaMemcpyAsync(ab + q_obig, obig.data(), obig.size() * 4, cudaMemcpyHostToDevice, st));
-      double *Y = (double *)(cb + p_y), *d_out = (double *)(ab + q_out);
+      CKT(cudaMemcpyAsync(ab, tab2.buf.data(), tab2.buf.size(), cudaMemcpyHostToDevice, st));
+      double *Y = (double *)(cb + p_y), *Z = (double *)(cb + p_z), *d_out = (double *)(ab + q_out);
       tc.dev = d_out;
       for (int b = 0; b < ngrp; ++b) max_kept = std::max(max_kept, grp[4 * b + 2]);
       select_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - sel0).count();
@@ -1514,42 +1860,63 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       {
         const int *d_oblk = (const int *)(ab + q_oblk), *d_obig = (const int *)(ab + q_obig);
         const int *d_grp = (const int *)(ab + q_grp), *d_k = (const int *)(ab + q_k);
+        int *d_first = (int *)(ab + q_first);
+        GemmParams g2;
+        std::memset(&g2, 0, sizeof g2);
+        g2.psi = Y;
+        g2.scr = (double *)(cb + p_g);
+        g2.out = (double *)(cb + p_g);
+        g2.cells = (const Cell *)(ab + q_cells);
+        g2.tasks = (const Task *)(ab + q_tasks);
+        g2.tiles = (const Tile *)(ab + q_gt);
+        g2.ntiles = (int)gtiles.size();
+        g2.counter = (unsigned int *)(ab + q_cnt);
+        launch_grouped_gemm(g2, grouped_gemm_grid(g2.ntiles), st);
+        const dim3 ogrid(ngrp, std::max(1, std::min(32, (max_kept + 7) / 8)));
+        ortho_check_kernel<<<ogrid, 256, 0, st>>>(d_grp, (const int64_t *)(ab + q_goff), (const double *)(cb + p_g), d_first);
+        ortho_factor_kernel<<<ogrid, 256, 0, st>>>(d_grp, (const int64_t *)(ab + q_goff), (double *)(cb + p_g), d_first);
+        g2.out = Z;
+        g2.tiles = (const Tile *)(ab + q_zt);
+        g2.ntiles = (int)ztiles.size();
+        g2.counter = (unsigned int *)(ab + q_cnt) + 1;
+        launch_grouped_gemm(g2, grouped_gemm_grid(g2.ntiles), st);
         if (ocl == 16) {
           CKT(cudaFuncSetAttribute(orthonormalize_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osm));
           orthonormalize_kernel<16><<<nocl * 16, ORTH_THREADS, osm, st>>>(d_oblk, d_obig, d_grp, d_dims, d_eoff, dev,
-                                                                          dinfo, d_k, Y, ldy, d_status);
+                                                                          dinfo, d_k, d_first, Z, ldy, d_status);
         } else {
           CKT(cudaFuncSetAttribute(orthonormalize_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osm));
           orthonormalize_kernel<8><<<nocl * 8, ORTH_THREADS, osm, st>>>(d_oblk, d_obig, d_grp, d_dims, d_eoff, dev,
-                                                                        dinfo, d_k, Y, ldy, d_status);
+                                                                        dinfo, d_k, d_first, Z, ldy, d_status);
         }
       }
       CKT(cudaGetLastError());
       CKT(cudaEventRecord(ctx->tev[6], st));
-      if (bt_reg) {
-        // eight reflectors per chunk: two CTAs fit an SM for sectors of up to 1536 states
-        const int kb = 8;
-        const size_t bsm = sizeof(double) * (size_t)kb * maxn;
-        const int rpl = (maxn + 31) / 32;
-        auto launch = [&](auto kern) -> cudaError_t {
-          cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm);
+      if (bt_wy) {
+        double *d_t = (double *)(ab + q_wyt);
+        if (npan) wy_t_kernel<<<npan, 256, 0, st>>>(ctx->trB.d(), d_roff, dtau, d_eoff, d_dims, (const int *)(ab + q_pan), d_t);
+        auto launch = [&](auto kern, int tiles, int vt) -> cudaError_t {
+          const int bsm = (int)sizeof(double) * bt_smem_doubles(tiles, vt);
+          cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm);
           if (e != cudaSuccess) return e;
-          kern<<<nslab, 32 * BT_WARPS, bsm, st>>>(ctx->trB.d(), d_roff, dtau, d_eoff, d_dims, (const int *)(ab + q_grp),
-                                                 (const int *)(ab + q_slab), Y, ldy, (const int64_t *)(ab + q_dst),
-                                                 d_out, kb);
+          kern<<<nslab, 32 * BT_WARPS, bsm, st>>>(ctx->trB.d(), d_roff, d_t, (const int *)(ab + q_pan0), d_dims,
+                                                  (const int *)(ab + q_grp), (const int *)(ab + q_slab), Z, ldy,
+                                                  (const int64_t *)(ab + q_dst), d_out);
           return cudaGetLastError();
         };
-        if (rpl <= 8) CKT(launch(backtransform_reg_kernel<8>));
-        else if (rpl <= 16) CKT(launch(backtransform_reg_kernel<16>));
-        else if (rpl <= 24) CKT(launch(backtransform_reg_kernel<24>));
-        else if (rpl <= 32) CKT(launch(backtransform_reg_kernel<32>));
-        else if (rpl <= 40) CKT(launch(backtransform_reg_kernel<40>));
-        else CKT(launch(backtransform_reg_kernel<48>));
+        // 128 states per row tile of a warp
+        if (maxn <= 128) CKT(launch(backtransform_wy_kernel<1, 2>, 1, 2));
+        else if (maxn <= 256) CKT(launch(backtransform_wy_kernel<2, 2>, 2, 2));
+        else if (maxn <= 512) CKT(launch(backtransform_wy_kernel<4, 2>, 4, 2));
+        else if (maxn <= 768) CKT(launch(backtransform_wy_kernel<6, 2>, 6, 2));
+        else if (maxn <= 1024) CKT(launch(backtransform_wy_kernel<8, 2>, 8, 2));
+        else if (maxn <= 1280) CKT(launch(backtransform_wy_kernel<10, 1>, 10, 1));
+        else CKT(launch(backtransform_wy_kernel<12, 1>, 12, 1));
       } else {
         const size_t bsm = sizeof(double) * (size_t)W * ldy;
         CKT(cudaFuncSetAttribute(backtransform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm));
         backtransform_kernel<<<nslab, 32 * W, bsm, st>>>(ctx->trB.d(), d_roff, dtau, d_eoff, d_dims,
-                                                         (const int *)(ab + q_grp), (const int *)(ab + q_slab), Y,
+                                                         (const int *)(ab + q_grp), (const int *)(ab + q_slab), Z,
                                                          ldy, (const int64_t *)(ab + q_dst), d_out);
         CKT(cudaGetLastError());
       }
