@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "hostutil.h"
 
 using namespace tjb;
 
@@ -135,21 +136,13 @@ static int upload_vec(tj_ctx *ctx, DevBuf &b, const std::vector<T> &v) {
   return TJ_OK;
 }
 
-static uint64_t fnv(uint64_t h, const void *p, size_t n) {
-  const unsigned char *c = (const unsigned char *)p;
-  for (size_t i = 0; i < n; ++i) {
-    h ^= c[i];
-    h *= 1099511628211ull;
-  }
-  return h;
-}
 static uint64_t key_block(uint64_t h, const tj_block &b) {
-  h = fnv(h, &b, sizeof b);
-  if (b.num > 0 && b.sub) h = fnv(h, b.sub, sizeof(tj_block_sub) * b.num);
+  h = key_bytes(h, &b, sizeof b);
+  if (b.num > 0 && b.sub) h = key_bytes(h, b.sub, sizeof(tj_block_sub) * b.num);
   return h;
 }
 static uint64_t key_model(uint64_t h, const tj_model *m) {
-  h = fnv(h, m, sizeof *m);
+  h = key_bytes(h, m, sizeof *m);
   h = key_block(h, m->ham);
   for (int i = 0; i < m->nsub; ++i) {
     const tj_block_set &s = m->sub[i];
@@ -158,27 +151,27 @@ static uint64_t key_model(uint64_t h, const tj_model *m) {
   return h;
 }
 static uint64_t key_basis(uint64_t h, const tj_basis *b) {
-  h = fnv(h, b, sizeof *b);
-  h = fnv(h, b->sub, sizeof(tj_basis_map) * b->num);
+  h = key_bytes(h, b, sizeof *b);
+  h = key_bytes(h, b->sub, sizeof(tj_basis_map) * b->num);
   int nm = 0;
   for (int i = 0; i < b->num; ++i) nm = std::max(nm, b->sub[i].first + b->sub[i].num);
-  return fnv(h, b->maps, sizeof(tj_basis_sub) * nm);
+  return key_bytes(h, b->maps, sizeof(tj_basis_sub) * nm);
 }
 static uint64_t key_lattice(uint64_t h, const tj_lattice *L) {
   const size_t ns1 = L->num_site + 1;
-  h = fnv(h, L, sizeof *L);
-  h = fnv(h, L->neib, sizeof(int32_t) * ns1 * L->neibt);
-  h = fnv(h, L->neiba, sizeof(int32_t) * ns1 * ns1);
-  h = fnv(h, L->inb1, sizeof(int32_t) * ns1 * ns1);
-  h = fnv(h, L->nleg11, sizeof(int32_t) * L->num_site);
-  h = fnv(h, L->nposi, sizeof(int32_t) * ns1);
-  h = fnv(h, L->nposi_dm, sizeof(int32_t) * ns1);
-  h = fnv(h, L->nposi_lat, sizeof(int32_t) * ns1);
-  h = fnv(h, L->jt, sizeof(double) * ns1 * L->neibt);
-  h = fnv(h, L->jz, sizeof(double) * ns1 * L->neibt);
-  h = fnv(h, L->jd, sizeof(double) * ns1 * L->neibt);
-  h = fnv(h, L->jn, sizeof(double) * L->neibt);
-  return fnv(h, L->esite, sizeof(double) * ns1);
+  h = key_bytes(h, L, sizeof *L);
+  h = key_bytes(h, L->neib, sizeof(int32_t) * ns1 * L->neibt);
+  h = key_bytes(h, L->neiba, sizeof(int32_t) * ns1 * ns1);
+  h = key_bytes(h, L->inb1, sizeof(int32_t) * ns1 * ns1);
+  h = key_bytes(h, L->nleg11, sizeof(int32_t) * L->num_site);
+  h = key_bytes(h, L->nposi, sizeof(int32_t) * ns1);
+  h = key_bytes(h, L->nposi_dm, sizeof(int32_t) * ns1);
+  h = key_bytes(h, L->nposi_lat, sizeof(int32_t) * ns1);
+  h = key_bytes(h, L->jt, sizeof(double) * ns1 * L->neibt);
+  h = key_bytes(h, L->jz, sizeof(double) * ns1 * L->neibt);
+  h = key_bytes(h, L->jd, sizeof(double) * ns1 * L->neibt);
+  h = key_bytes(h, L->jn, sizeof(double) * L->neibt);
+  return key_bytes(h, L->esite, sizeof(double) * ns1);
 }
 
 static uint64_t instance_key(uint64_t h, const tj_lattice *lat, const tj_model *sys, const tj_model *env,
@@ -188,7 +181,7 @@ static uint64_t instance_key(uint64_t h, const tj_lattice *lat, const tj_model *
   h = key_model(h, env);
   h = key_basis(h, sys_bs);
   h = key_basis(h, env_bs);
-  return fnv(h, wave->sub, sizeof(tj_wave_sub) * wave->num);
+  return key_bytes(h, wave->sub, sizeof(tj_wave_sub) * wave->num);
 }
 
 // Compiles (or reuses) the plan of H*psi and uploads operators and work lists.
@@ -198,8 +191,8 @@ int tjb::prepare_hpsi(tj_ctx *ctx, const tj_lattice *lat, const tj_model *sys, c
   if (!lat->neib || !lat->nleg11 || !lat->jt || !sys->sub || !env->sub || !sys_bs->sub || !env_bs->sub || !wave->sub)
     return set_err(TJ_ERR_ARG, "null table in the inputs");
   uint64_t h = instance_key(1469598103934665603ull, lat, sys, env, sys_bs, env_bs, wave);
-  h = fnv(h, &ctx->prec_mode, sizeof ctx->prec_mode);
-  h = fnv(h, &ctx->slices, sizeof ctx->slices);
+  h = key_bytes(h, &ctx->prec_mode, sizeof ctx->prec_mode);
+  h = key_bytes(h, &ctx->slices, sizeof ctx->slices);
   if (ctx->plan_valid && ctx->plan_key == h && tune_is_current(ctx)) return reset_device_flags(ctx);
   ctx->plan_valid = false;
   CK(cudaSetDevice(ctx->device));
@@ -534,9 +527,9 @@ extern "C" int tj_model_wave_multi(tj_ctx *ctx, int n, const tj_lattice *const *
     if (!same_layout(invec[i], outvec[i])) return set_err(TJ_ERR_ARG, "outvec must have invec's sector layout");
     h = instance_key(h, lat[i], sys[i], env[i], sys_bs[i], env_bs[i], invec[i]);
   }
-  h = fnv(h, &n, sizeof n);
-  h = fnv(h, &ctx->prec_mode, sizeof ctx->prec_mode);
-  h = fnv(h, &ctx->slices, sizeof ctx->slices);
+  h = key_bytes(h, &n, sizeof n);
+  h = key_bytes(h, &ctx->prec_mode, sizeof ctx->prec_mode);
+  h = key_bytes(h, &ctx->slices, sizeof ctx->slices);
   CK(cudaSetDevice(ctx->device));
   if (!(ctx->plan_valid && ctx->plan_key == h && tune_is_current(ctx) && (int)ctx->multi_off.size() == n)) {
     ctx->plan_valid = false;

@@ -11,7 +11,6 @@
 // transposed view only flips the operand's transpose flag.
 #include <algorithm>
 #include <functional>
-#include <unordered_set>
 #include <array>
 #include <climits>
 #include <cmath>
@@ -22,6 +21,7 @@
 #include <tuple>
 #include <unordered_map>
 
+#include "hostutil.h"
 #include "tj_internal.h"
 
 int tjb_set_err(int code, const std::string &m);
@@ -70,7 +70,7 @@ double w3j(int j1, int j2, int j3, int m1, int m2, int m3) {
   return ((ph % 2) ? -1.0 : 1.0) * std::sqrt(tri * mf) * sum;
 }
 
-double w6j(int j1, int j2, int j3, int l1, int l2, int l3) {
+static double w6j_sum(int j1, int j2, int j3, int l1, int l2, int l3) {
   if (!g_fact_ready) {
     std::fill(g_fact, g_fact + 302, 0.0);
     g_fact[0] = 1.0;
@@ -100,6 +100,24 @@ double w6j(int j1, int j2, int j3, int l1, int l2, int l3) {
   return omega * std::sqrt(t1 * t2 * t3 * t4);
 }
 
+// The symbols met before, per thread, in a direct-mapped table (64 KB): a plan
+// asks for a few hundred different ones some 10^5 times, and the factorial sum
+// takes 100 ns.
+double w6j(int j1, int j2, int j3, int l1, int l2, int l3) {
+  if ((unsigned)(j1 | j2 | j3 | l1 | l2 | l3) > 1023u) return w6j_sum(j1, j2, j3, l1, l2, l3);
+  struct Slot {
+    uint64_t key = 0;
+    double v = 0;
+  };
+  constexpr int BITS = 12;
+  static thread_local std::vector<Slot> table;
+  if (table.empty()) table.resize(1 << BITS);
+  const uint64_t key = 1 + ((((((uint64_t)j1 << 10 | j2) << 10 | j3) << 10 | l1) << 10 | l2) << 10 | l3);
+  Slot &s = table[(key * 0x9e3779b97f4a7c15ull) >> (64 - BITS)];
+  if (s.key != key) s = Slot{key, w6j_sum(j1, j2, j3, l1, l2, l3)};
+  return s.v;
+}
+
 namespace {
 
 struct PlanError : std::runtime_error {
@@ -117,7 +135,18 @@ struct OSub {
 };
 struct OBlk {
   int len = 0, up_dif = 0, down_dif = 0;
-  std::vector<OSub> sub;
+  std::vector<OSub> sub;          // complete before the first search
+  mutable LabelIndex by_label[2];  // of (num_up, num_down), and with down_dif; made at the first search
+  int find(int nu, int nd, int dd, bool use_dd) const {
+    LabelIndex &ix = by_label[use_dd];
+    if (!ix.built())
+      ix.build((int)sub.size(), [&](int k, int *l) {
+        l[0] = sub[k].num_up;
+        l[1] = sub[k].num_down;
+        l[2] = use_dd ? sub[k].down_dif : 0;
+      });
+    return ix.find(nu, nd, use_dd ? dd : 0);
+  }
 };
 // A block, or its transpose (block_transfer_trans) without copying.
 struct OView {
@@ -146,6 +175,8 @@ struct OView {
   }
   // first sub-block with the labels (num_up, num_down[, down_dif])
   int find(int nu_, int nd_, int dd_, bool use_dd) const {
+    if (!tr) return b->find(nu_, nd_, dd_, use_dd);
+    if (use_dd) return b->find(nu_ - b->up_dif, nd_ + dd_, -dd_, true);   // the labels of the stored matrix
     for (int k = 0; k < num(); ++k)
       if (nu(k) == nu_ && nd(k) == nd_ && (!use_dd || dd(k) == dd_)) return k;
     return -1;
@@ -239,10 +270,10 @@ void split_tiles(const std::vector<Cell> &cells, const std::vector<Task> &tasks,
   // tiles in emission order with their weights; sorted below by weight,
   // heaviest first, ties kept in emission order
   std::vector<Tile> all;
-  std::vector<std::pair<double, int64_t>> w;
+  std::vector<uint64_t> w;
   all.reserve((size_t)ntile + cells.size());
   w.reserve((size_t)ntile + cells.size());
-  std::vector<double> chunk_w;
+  std::vector<uint64_t> chunk_w;
   std::vector<std::pair<int, int>> chunks;
   for (int ci = 0; ci < (int)cells.size(); ++ci) {
     const Cell &c = cells[ci];
@@ -261,7 +292,7 @@ void split_tiles(const std::vector<Cell> &cells, const std::vector<Task> &tasks,
     }
     chunks.push_back({start, ge});
     const bool split = chunks.size() > 1 && !dot_mode;
-    chunk_w.assign(chunks.size(), 1.0);
+    chunk_w.assign(chunks.size(), 1);
     for (size_t k = 0; k < chunks.size(); ++k)
       for (int t = chunks[k].first; t < chunks[k].second; ++t) chunk_w[k] += tasks[t].K;
     for (int r = 0; r < c.M; r += BM)
@@ -283,26 +314,27 @@ void split_tiles(const std::vector<Cell> &cells, const std::vector<Task> &tasks,
           t.ab = ge;
           t.ae = (!split && k == 0) ? c.t_end : ge;
           t.slot = split ? slot0 + (int)k : -1;
-          w.push_back({chunk_w[k], (int64_t)all.size()});
+          w.push_back(chunk_w[k]);
           all.push_back(t);
         }
       }
   }
-  // the weights take few distinct values: a stable counting sort over their
-  // ranks (heaviest first) gives the order of a stable sort by weight
-  std::unordered_set<double> distinct;
-  for (auto &p : w) distinct.insert(p.first);
-  std::vector<double> uniq(distinct.begin(), distinct.end());
-  std::sort(uniq.begin(), uniq.end(), std::greater<double>());
-  std::vector<int64_t> start(uniq.size() + 1, 0);
-  std::vector<int32_t> rank(w.size());
-  for (size_t j = 0; j < w.size(); ++j) {
-    rank[j] = (int32_t)(std::lower_bound(uniq.begin(), uniq.end(), w[j].first, std::greater<double>()) - uniq.begin());
-    ++start[rank[j] + 1];
+  // heaviest first, ties in emission order: a radix sort of the weights'
+  // distances from the largest, 11 bits a pass
+  uint64_t most = 0;
+  for (uint64_t x : w) most = std::max(most, x);
+  std::vector<uint32_t> order(w.size()), next(w.size());
+  for (size_t j = 0; j < w.size(); ++j) order[j] = (uint32_t)j;
+  for (int shift = 0; shift < 64 && (most >> shift) != 0; shift += 11) {
+    size_t start[2049] = {0};
+    auto digit = [&](uint32_t j) { return (size_t)(((most - w[j]) >> shift) & 2047); };
+    for (uint32_t j : order) ++start[digit(j) + 1];
+    for (int r = 0; r < 2048; ++r) start[r + 1] += start[r];
+    for (uint32_t j : order) next[start[digit(j)]++] = j;
+    order.swap(next);
   }
-  for (size_t r = 0; r < uniq.size(); ++r) start[r + 1] += start[r];
   tiles.resize(all.size());
-  for (size_t j = 0; j < w.size(); ++j) tiles[start[rank[j]]++] = all[w[j].second];
+  for (size_t j = 0; j < order.size(); ++j) tiles[j] = all[order[j]];
 }
 
 namespace {
@@ -336,7 +368,7 @@ struct Builder {
       return (size_t)h;
     }
   };
-  std::unordered_map<ProdKey, int, ProdKeyHash> prod_id;
+  FlatMap<ProdKey, int, ProdKeyHash> prod_id{1 << 13};
   bool dedup = true;
   bool cor_mode = false;   // correlators: keep only the cells that have tasks
   bool want_tiles = true;  // make the FP64 work lists
@@ -417,7 +449,7 @@ struct Builder {
     // so that the lists are not regrown and rehashed while the terms are emitted
     out_tasks.reserve((size_t)ncells * 4);
     out_cell.reserve((size_t)ncells * 4);
-    prod_id.reserve((size_t)ncells * 2);
+    prod_id = FlatMap<ProdKey, int, ProdKeyHash>((size_t)ncells * 4 + 16);
     plan.cells1.reserve((size_t)ncells * 2);
     plan.tasks1.reserve((size_t)ncells * 2);
     plan.cell1_row_state.reserve((size_t)ncells * 2);
@@ -508,12 +540,12 @@ struct Builder {
     Operand a = A.mat(ka, at);
     const ProdKey key{a.off, xc, (int32_t)a.trans};
     int pid;
-    auto it = dedup ? prod_id.find(key) : prod_id.end();
-    if (it != prod_id.end()) {
-      pid = it->second;
+    const int *known = dedup ? prod_id.find(key) : nullptr;
+    if (known) {
+      pid = *known;
     } else {
       pid = (int)plan.cells1.size();
-      if (dedup) prod_id[key] = pid;
+      if (dedup) prod_id.emplace(key, pid);
       Cell c;
       std::memset(&c, 0, sizeof c);
       c.off = plan.scratch_len;
@@ -1114,6 +1146,7 @@ static void load_block(const tj_block &b, OBlk &o, HpsiPlan &plan) {
   o.up_dif = b.up_dif;
   o.down_dif = b.down_dif;
   o.sub.clear();
+  for (LabelIndex &ix : o.by_label) ix = LabelIndex();
   if (b.num < 0 || (b.num > 0 && (!b.sub || !b.data))) throw PlanError(TJ_ERR_ARG, "block with null sub/data");
   // one host-to-device copy per block: the span of its sub-block matrices
   int64_t lo = LLONG_MAX, hi = 0;

@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "hostutil.h"
 
 using namespace tjb;
 
@@ -94,22 +95,34 @@ struct EBlk {
   int len = 0, up_dif = 0, down_dif = 0;
   bool set = false;   // holds an operator (slots of the reference's next%sub)
   std::vector<ESub> sub;
-  int find(int nu, int nd, int dd, bool use_dd) const {
-    for (size_t k = 0; k < sub.size(); ++k)
-      if (sub[k].num_up == nu && sub[k].num_down == nd && (!use_dd || sub[k].down_dif == dd)) return (int)k;
-    return -1;
-  }
 };
 
 inline double m1(int n) { return (n % 2) ? -1.0 : 1.0; }   // (-1)**n
 inline double fsign(char flag, int n) { return flag == 'F' ? m1(n) : 1.0; }
 
+// index of a block's sub-blocks by their labels; use_dd: down_dif among them
+template <class S>
+LabelIndex label_index(const std::vector<S> &sub, bool use_dd) {
+  LabelIndex ix;
+  ix.build((int)sub.size(), [&](int k, int *l) {
+    l[0] = sub[k].num_up;
+    l[1] = sub[k].num_down;
+    l[2] = use_dd ? sub[k].down_dif : 0;
+  });
+  return ix;
+}
+
 struct Ctx {
   const tj_basis *bs;
+  mutable LabelIndex by_label;   // of bs, made at the first search
   int find_bs(int nu, int nd) const {
-    for (int x = 0; x < bs->num; ++x)
-      if (bs->sub[x].new_num_up == nu && bs->sub[x].new_num_down == nd) return x;
-    return -1;
+    if (!by_label.built())
+      by_label.build(bs->num, [&](int k, int *l) {
+        l[0] = bs->sub[k].new_num_up;
+        l[1] = bs->sub[k].new_num_down;
+        l[2] = 0;
+      });
+    return by_label.find(nu, nd, 0);
   }
   const tj_basis_sub &M(int x, int m) const { return bs->maps[bs->sub[x].first + m]; }
 };
@@ -119,12 +132,15 @@ EBlk enl_dia(const Ctx &c, const RBlk *blk, const SiteOp *site) {
   EBlk e;
   e.len = c.bs->len;
   e.set = true;
+  e.sub.reserve(c.bs->num);
+  const LabelIndex bix = blk ? label_index(blk->sub, false) : LabelIndex();
   for (int k = 0; k < c.bs->num; ++k) {
     ESub s{c.bs->sub[k].new_num_up, c.bs->sub[k].new_num_down, 0, k, k, {}};
+    s.p.reserve(c.bs->sub[k].num);
     for (int x = 0; x < c.bs->sub[k].num; ++x) {
       const tj_basis_sub &m = c.M(k, x);
       if (blk) {
-        const int i = blk->find(m.bl_num_up, m.bl_num_down, 0, false);
+        const int i = bix.find(m.bl_num_up, m.bl_num_down, 0);
         if (i < 0) continue;
         const RSub &o = blk->sub[i];
         if (o.row_dim != m.sdim || o.sdim != m.sdim)
@@ -152,19 +168,22 @@ EBlk enl_ndia(const Ctx &c, const RBlk *blk, const SiteOp *site, bool env_side, 
   e.up_dif = blk ? blk->up_dif : site->up_dif;
   e.down_dif = blk ? blk->down_dif : site->down_dif;
   const int up_dif = e.up_dif, d1 = e.down_dif;
+  e.sub.reserve((size_t)c.bs->num * (d1 + 1));
+  const LabelIndex bix = blk ? label_index(blk->sub, true) : LabelIndex();
   for (int x = 0; x < c.bs->num; ++x)
     for (int dd = -d1; dd <= d1; dd += 2) {
       const int rnu = c.bs->sub[x].new_num_up, rnd = c.bs->sub[x].new_num_down;
       const int y = c.find_bs(rnu + up_dif, rnd + dd);
       if (y < 0) continue;
       ESub s{rnu, rnd, dd, y, x, {}};
+      s.p.reserve(4);
       const int lnd = rnd + dd;
       for (int q = 0; q < c.bs->sub[x].num; ++q) {
         const tj_basis_sub &m = c.M(x, q);
         for (int sdd = -d1; sdd <= d1; sdd += 2) {
           const tj_basis_sub *ml = nullptr;
           if (blk) {
-            const int bid = blk->find(m.bl_num_up, m.bl_num_down, sdd, true);
+            const int bid = bix.find(m.bl_num_up, m.bl_num_down, sdd);
             if (bid < 0) continue;
             const int lsnu = m.bl_num_up + up_dif, lsnd = m.bl_num_down + sdd;
             for (int r = 0; r < c.bs->sub[y].num && !ml; ++r) {
@@ -206,13 +225,14 @@ EBlk enl_ndia(const Ctx &c, const RBlk *blk, const SiteOp *site, bool env_side, 
 // Get_hamiltonian_ndia (get_sys.f90:578-759): coef [block x site^T + h.c.]
 void ham_ndia(const Ctx &c, const RBlk &blk, const SiteOp &site, double coef, EBlk &ham, char flagsign, bool sys_side) {
   const int up_dif = blk.up_dif, d1 = blk.down_dif;
+  const LabelIndex bix = label_index(blk.sub, true);
   for (ESub &h : ham.sub) {
     const int rnd = h.num_down;
     const int x = h.rsec, y = h.lsec;
     for (int q = 0; q < c.bs->sub[x].num; ++q) {
       const tj_basis_sub &m = c.M(x, q);
       for (int sdd = -d1; sdd <= d1; sdd += 2) {
-        const int bid = blk.find(m.bl_num_up, m.bl_num_down, sdd, true);
+        const int bid = bix.find(m.bl_num_up, m.bl_num_down, sdd);
         if (bid < 0) continue;
         const int lsnu = m.bl_num_up + up_dif, lsnd = m.bl_num_down + sdd;
         for (int nsd = std::abs(m.st_num_down - site.down_dif); nsd <= m.st_num_down + site.down_dif; nsd += 2) {
@@ -246,8 +266,9 @@ void ham_ndia(const Ctx &c, const RBlk &blk, const SiteOp &site, double coef, EB
 // site operator enlarged by update_block_dia / update_site_dia (both
 // block-diagonal over the basis's sub-sectors, o2 a multiple of I on each)
 void ham_dia(const EBlk &o1, const EBlk &o2, double coef, EBlk &ham) {
+  const LabelIndex i1 = label_index(o1.sub, false), i2 = label_index(o2.sub, false);
   for (ESub &h : ham.sub) {
-    const int a = o1.find(h.num_up, h.num_down, 0, false), b = o2.find(h.num_up, h.num_down, 0, false);
+    const int a = i1.find(h.num_up, h.num_down, 0), b = i2.find(h.num_up, h.num_down, 0);
     if (a < 0 || b < 0) continue;
     const double c1 = coef / std::sqrt(1.0 + h.num_down);
     for (const Piece &p1 : o1.sub[a].p)
@@ -285,11 +306,6 @@ struct TSec {
 };
 struct TBlk {
   std::vector<TSec> sec;
-  int find(int nu, int nd) const {
-    for (size_t k = 0; k < sec.size(); ++k)
-      if (sec[k].num_up == nu && sec[k].num_down == nd) return (int)k;
-    return -1;
-  }
 };
 
 // output sub-block records, in the order of the result
@@ -326,7 +342,7 @@ struct Builder {
       return (size_t)h;
     }
   };
-  std::unordered_map<Key, int64_t, KeyHash> prod;   // phase-1 product -> its scratch offset
+  FlatMap<Key, int64_t, KeyHash> prod{8192};   // phase-1 product -> its scratch offset
   std::vector<Task> t2;
   std::vector<int32_t> t2cell;
 
@@ -335,8 +351,7 @@ struct Builder {
   int64_t product(const Operand &Lop, const Operand &Rop, int M, int N, int K, int8_t assoc) {
     Key key{Lop.space == SP_OPS ? Lop.off : Rop.off, Lop.space == SP_OPS ? Rop.off : Lop.off, M, N, K,
             Lop.trans, Rop.trans, assoc};
-    auto it = prod.find(key);
-    if (it != prod.end()) return it->second;
+    if (const int64_t *at = prod.find(key)) return *at;
     const int64_t off = P.scratch_len;
     P.scratch_len += (int64_t)M * N;
     P.scratch_len = (P.scratch_len + 3) / 4 * 4;
@@ -441,19 +456,26 @@ struct Builder {
       recs.push_back(r);
       ob.num++;
     };
+    const LabelIndex eix = label_index(e.sub, !dia);
     if (dia) {
       for (size_t i = 0; i < trun.sec.size(); ++i) {
-        const int x = e.find(trun.sec[i].num_up, trun.sec[i].num_down, 0, false);
+        const int x = eix.find(trun.sec[i].num_up, trun.sec[i].num_down, 0);
         add(x >= 0 ? &e.sub[x] : nullptr, (int)i, (int)i, 0);
       }
       ob.dim = trun_dim;
     } else {
       const int d1 = e.down_dif;
+      LabelIndex tix;
+      tix.build((int)trun.sec.size(), [&](int k, int *l) {
+        l[0] = trun.sec[k].num_up;
+        l[1] = trun.sec[k].num_down;
+        l[2] = 0;
+      });
       for (size_t x = 0; x < trun.sec.size(); ++x)
         for (int dd = -d1; dd <= d1; dd += 2) {
-          const int y = trun.find(trun.sec[x].num_up + e.up_dif, trun.sec[x].num_down + dd);
+          const int y = tix.find(trun.sec[x].num_up + e.up_dif, trun.sec[x].num_down + dd, 0);
           if (y < 0) continue;
-          const int o = e.find(trun.sec[x].num_up, trun.sec[x].num_down, dd, true);
+          const int o = eix.find(trun.sec[x].num_up, trun.sec[x].num_down, dd);
           add(o >= 0 ? &e.sub[o] : nullptr, y, (int)x, dd);
           ob.dim += trun.sec[x].kept;
         }
@@ -618,12 +640,28 @@ int build_renorm_plan(const tj_lattice *lat, int side, int mshift, const tj_mode
       }
       const int jn = INB1(len0 + 1, len0 + 1);
       if (jn < 1 || jn >= nslot) throw RenormError(TJ_ERR_ARG, "new site has no operator slot");
-      next[jn][kinds[0]] = tmp;
-      if (ij == 1) next[jn][1] = tmp1;
+      next[jn][kinds[0]] = std::move(tmp);
+      if (ij == 1) next[jn][1] = std::move(tmp1);
       for (int ii = 1; ii <= nl1; ++ii)
-        for (int q = 0; q < nk; ++q) keep[ii][kinds[q]] = next[ii][kinds[q]];
+        for (int q = 0; q < nk; ++q) keep[ii][kinds[q]] = std::move(next[ii][kinds[q]]);   // read no more here
     }
     // truncated output, in result order: ham, then each set's five operators
+    {   // capacities: a few pieces per sub-block
+      size_t np = 0, ns = 0;
+      auto count = [&](const EBlk &e) {
+        ns += e.sub.size();
+        for (const ESub &q : e.sub) np += q.p.size();
+      };
+      count(nham);
+      for (const auto &k : keep)
+        for (const EBlk &e : k) count(e);
+      B.t2.reserve(np);
+      B.t2cell.reserve(np);
+      P.tasks1.reserve(np);
+      P.cells1.reserve(np);
+      P.cells2.reserve(ns);
+      B.recs.reserve(ns);
+    }
     B.truncate(nham, true, len0 + 1);
     for (int ii = 1; ii <= nl1; ++ii) {
       B.truncate(keep[ii][0], false, len0 + 1);
@@ -709,17 +747,9 @@ std::shared_ptr<tj_renorm_state> tjb::new_renorm_state() { return std::make_shar
 
 namespace {
 
-uint64_t fnv(uint64_t h, const void *p, size_t n) {
-  const unsigned char *c = (const unsigned char *)p;
-  for (size_t i = 0; i < n; ++i) {
-    h ^= c[i];
-    h *= 1099511628211ull;
-  }
-  return h;
-}
 uint64_t key_block(uint64_t h, const tj_block &b) {
-  h = fnv(h, &b, sizeof b);
-  if (b.num > 0 && b.sub) h = fnv(h, b.sub, sizeof(tj_block_sub) * b.num);
+  h = key_bytes(h, &b, sizeof b);
+  if (b.num > 0 && b.sub) h = key_bytes(h, b.sub, sizeof(tj_block_sub) * b.num);
   return h;
 }
 // structural key of a renormalisation call: tables and data pointers (the
@@ -727,17 +757,17 @@ uint64_t key_block(uint64_t h, const tj_block &b) {
 uint64_t renorm_key(const tj_lattice *lat, int side, int mshift, const tj_model *pre, const tj_basis *basis,
                     const tj_block *trun) {
   uint64_t h = 1469598103934665603ull;
-  h = fnv(h, lat, sizeof *lat);
-  h = fnv(h, &side, sizeof side);
-  h = fnv(h, &mshift, sizeof mshift);
-  h = fnv(h, pre, sizeof *pre);
+  h = key_bytes(h, lat, sizeof *lat);
+  h = key_bytes(h, &side, sizeof side);
+  h = key_bytes(h, &mshift, sizeof mshift);
+  h = key_bytes(h, pre, sizeof *pre);
   h = key_block(h, pre->ham);
   for (int i = 0; i < pre->nsub && pre->sub; ++i) {
     const tj_block_set &s = pre->sub[i];
     h = key_block(key_block(key_block(key_block(h, s.elec_up), s.elec_down), s.spin_sd), s.num_sn);
   }
-  h = fnv(h, basis, sizeof *basis);
-  if (basis->sub) h = fnv(h, basis->sub, sizeof(tj_basis_map) * basis->num);
+  h = key_bytes(h, basis, sizeof *basis);
+  if (basis->sub) h = key_bytes(h, basis->sub, sizeof(tj_basis_map) * basis->num);
   return key_block(h, *trun);
 }
 
@@ -1178,9 +1208,9 @@ int carry_dev(tj_ctx *ctx, const tj_chain *ch, int side, bool dia, char types, D
 }
 
 uint64_t key_chain(uint64_t h, const tj_chain *ch) {
-  h = fnv(h, ch, sizeof *ch);
-  if (ch->bsm && ch->n > 0) h = fnv(h, ch->bsm, sizeof(tj_basis) * ch->n);
-  if (ch->truns && ch->n > 0) h = fnv(h, ch->truns, sizeof(tj_block) * ch->n);
+  h = key_bytes(h, ch, sizeof *ch);
+  if (ch->bsm && ch->n > 0) h = key_bytes(h, ch->bsm, sizeof(tj_basis) * ch->n);
+  if (ch->truns && ch->n > 0) h = key_bytes(h, ch->truns, sizeof(tj_block) * ch->n);
   return h;
 }
 
@@ -1223,8 +1253,8 @@ extern "C" int tj_get_oper(tj_ctx *ctx, int side, int dia, const tj_chain *chain
     return set_err(TJ_ERR_ARG, "tj_get_oper: bad argument");
   uint64_t h = 1469598103934665603ull;
   const int args[6] = {1, side, dia, old_idx, new_idx, truns};
-  h = fnv(h, args, sizeof args);
-  h = fnv(h, &types, 1);
+  h = key_bytes(h, args, sizeof args);
+  h = key_bytes(h, &types, 1);
   h = key_block(h, *st_oper);
   h = key_chain(h, chain);
   return meas_call(ctx, h, out, [&](DevOp &res, std::string &msg) -> int {
@@ -1278,8 +1308,8 @@ extern "C" int tj_change_oper(tj_ctx *ctx, int side, int dia, const tj_chain *ch
     return set_err(TJ_ERR_ARG, "tj_change_oper: bad argument");
   uint64_t h = 1469598103934665603ull;
   const int args[6] = {2, side, dia, old_idx, new_idx, truns};
-  h = fnv(h, args, sizeof args);
-  h = fnv(h, &types, 1);
+  h = key_bytes(h, args, sizeof args);
+  h = key_bytes(h, &types, 1);
   h = key_block(h, *old_oper);
   h = key_chain(h, chain);
   return meas_call(ctx, h, out, [&](DevOp &res, std::string &msg) -> int {
@@ -1299,7 +1329,7 @@ extern "C" int tj_update_trun(tj_ctx *ctx, int dia, const tj_block *ori, const t
   if (!ori || !trun) return set_err(TJ_ERR_ARG, "tj_update_trun: null argument");
   uint64_t h = 1469598103934665603ull;
   const int args[2] = {3, dia};
-  h = fnv(h, args, sizeof args);
+  h = key_bytes(h, args, sizeof args);
   h = key_block(key_block(h, *ori), *trun);
   return meas_call(ctx, h, out, [&](DevOp &res, std::string &msg) -> int {
     DevOp cur;
@@ -1320,13 +1350,13 @@ extern "C" int tj_block_mul_block_ndia(tj_ctx *ctx, const tj_block *oper1, char 
     return set_err(TJ_ERR_ARG, "tj_block_mul_block_ndia: flags must be 'N' or 'T'");
   uint64_t h = 1469598103934665603ull;
   const int args[2] = {4, down_dif};
-  h = fnv(h, args, sizeof args);
-  h = fnv(h, &flag1, 1);
-  h = fnv(h, &flag2, 1);
-  h = fnv(h, &coef, sizeof coef);
+  h = key_bytes(h, args, sizeof args);
+  h = key_bytes(h, &flag1, 1);
+  h = key_bytes(h, &flag2, 1);
+  h = key_bytes(h, &coef, sizeof coef);
   h = key_block(key_block(h, *oper1), *oper2);
-  h = fnv(h, basis, sizeof *basis);
-  h = fnv(h, basis->sub, sizeof(tj_basis_map) * basis->num);
+  h = key_bytes(h, basis, sizeof *basis);
+  h = key_bytes(h, basis->sub, sizeof(tj_basis_map) * basis->num);
   return meas_call(ctx, h, out, [&](DevOp &res, std::string &msg) -> int {
     HpsiPlan P;
     RBlk a, b;

@@ -36,13 +36,13 @@ int ilog2(int64_t x) {
 }  // namespace
 
 uint64_t plan_hist_key(const HpsiPlan &P, int prec_mode, int slices) {
-  std::map<uint32_t, int64_t> hist;
+  // counted in an array, read out in the order of the packed logarithms
+  std::vector<int32_t> hist(1 << 15, 0);
   auto count = [&](const std::vector<Cell> &cells, const std::vector<Task> &tasks) {
     for (const Cell &c : cells)
       for (int t = c.t_begin; t < c.t_end; ++t) {
         if (tasks[t].R.space == SP_NONE) continue;
-        const uint32_t b = (uint32_t)ilog2(c.M) | ((uint32_t)ilog2(c.N) << 8) | ((uint32_t)ilog2(tasks[t].K) << 16);
-        ++hist[b];
+        ++hist[(uint32_t)ilog2(c.M) | ((uint32_t)ilog2(c.N) << 5) | ((uint32_t)ilog2(tasks[t].K) << 10)];
       }
   };
   count(P.cells1, P.tasks1);
@@ -56,10 +56,11 @@ uint64_t plan_hist_key(const HpsiPlan &P, int prec_mode, int slices) {
   };
   mix((uint64_t)prec_mode);
   mix((uint64_t)(prec_mode == TJ_PREC_OZAKI ? slices : 0));
-  for (const auto &kv : hist) {
-    mix(kv.first);
-    mix((uint64_t)kv.second);
-  }
+  for (uint32_t b = 0; b < hist.size(); ++b)
+    if (hist[b]) {
+      mix((b & 31) | (b >> 5 & 31) << 8 | (uint64_t)(b >> 10) << 16);
+      mix((uint64_t)hist[b]);
+    }
   return h;
 }
 
