@@ -56,7 +56,14 @@ tj_ctx::~tj_ctx() {
   for (auto &e : tev)
     if (e) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
+  if (side) cudaStreamDestroy(side);
   if (pinned) cudaFreeHost(pinned);
+}
+
+int tj_ctx::side_stream(cudaStream_t &s) {
+  if (!side) CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  s = side;
+  return TJ_OK;
 }
 
 extern "C" int tj_ctx_create(tj_ctx **out, int device) {
@@ -395,16 +402,21 @@ static int run_hpsi_oz(tj_ctx *ctx, const double *in, double *out, bool timed) {
   return TJ_OK;
 }
 
+// The error of the split-precision kernels' device flags.
+static int report_flags(int flag) {
+  if (flag & 2)
+    return set_err(TJ_ERR_NUMERIC, "split-precision H*psi: the input vector (or a product) holds a NaN or an infinity");
+  if (flag & 1) return set_err(TJ_ERR_TIMEOUT, "split-precision GEMM: a bounded tensor-core wait timed out");
+  return TJ_OK;
+}
+
 // Reads the device error flag of the split-precision kernels (bounded waits).
 int tjb::check_device_flags(tj_ctx *ctx) {
   if (!ctx->oz) return TJ_OK;
   int flag = 0;
   CK(cudaMemcpyAsync(&flag, (char *)ctx->ozMisc.p + 64, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (flag & 2)
-    return set_err(TJ_ERR_NUMERIC, "split-precision H*psi: the input vector (or a product) holds a NaN or an infinity");
-  if (flag & 1) return set_err(TJ_ERR_TIMEOUT, "split-precision GEMM: a bounded tensor-core wait timed out");
-  return TJ_OK;
+  return report_flags(flag);
 }
 
 // Clears the split-precision kernels' error flags at the start of a call, so
@@ -625,10 +637,10 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   const int64_t ld = (D + 31) / 32 * 32;
   if ((rc = ctx->lanV.reserve(sizeof(double) * ld * (LOOP_IN + 4)))) return rc;
   const int nblk = dot_blocks(D);
-  const int mdb = (int)((D + 256 * 8 - 1) / (256 * 8));
+  const int mdb = lz_slices(D);
   if ((rc = ctx->lanScal.reserve(sizeof(double) * 1024))) return rc;
   const int npart = std::max(nblk, lz_blocks(D));
-  if ((rc = ctx->lanPart.reserve(sizeof(double) * ((size_t)std::max(npart, 1) + (size_t)std::max(mdb, 1) * 128 + 256))))
+  if ((rc = ctx->lanPart.reserve(sizeof(double) * ((size_t)std::max(npart, 1) + (size_t)mdb * 129 + 256))))
     return rc;
   double *V = ctx->lanV.d();
   double *S = ctx->lanScal.d();   // [0..127] alpha, [128..255] beta, [256..383] uu, [384..511] coef, [512] lam, [513] nrm, [600..727] dz
@@ -674,16 +686,25 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   // computed speculatively and dropped, with `last` restored, so the result
   // is the same.
   auto ref = [&](int off) { return LzRef{V, ld, itd, off, nullptr}; };
+  const bool is_short = lz_short(D);
+  cudaStream_t side = nullptr;
+  if (is_short && (rc = ctx->side_stream(side))) return rc;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-  launch_lz_update_norm(ref(1), Y, ref(0), ref(-1), S, itd, D, part, cnt, st);   // vec(L+1), beta(L)
-  launch_lz_gram_schmidt(V, ld, itd, ref(1), D, S, mpart, mdb, 128, uu + 1, coef, part, cnt, st);
-  launch_lz_scale_norm(ref(1), X, D, S, itd, part, cnt, st);                    // X = vec(L+1), uu(L+1)
+  const int *err = ctx->oz ? (const int *)((char *)ctx->ozMisc.p + 64) : nullptr;
+  if (is_short) {
+    launch_lz_step_short(V, ld, itd, Y, X, D, S, st);
+  } else {
+    launch_lz_update_gram_schmidt(V, ld, itd, ref(1), Y, D, S, mpart, 128, uu + 1, coef, part, cnt, st);   // vec(L+1), beta(L)
+    launch_lz_scale_norm(ref(1), X, D, S, itd, part, cnt, st);                    // X = vec(L+1), uu(L+1)
+  }
   rc = run_hpsi(ctx, X, Y, false);
-  if (!rc) {
-    launch_lz_dot(ref(1), Y, D, S, itd, part, cnt, st);                         // alpha(L+1)
-    launch_lz_tridiag_publish(S, itd, ctx->pinned, st);
+  if (!rc && is_short) {
+    launch_lz_dot_short(X, Y, D, S, itd, err, st);
+  } else if (!rc) {
+    launch_lz_dot(ref(1), Y, D, S, itd, part, cnt, st);                           // alpha(L+1)
+    launch_lz_tridiag_publish(S, itd, err, ctx->pinned, st);
   }
   const cudaError_t ce = cudaStreamEndCapture(st, &graph);
   --ctx->n_hpsi;   // the captured H*psi ran nothing
@@ -697,14 +718,36 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   if (ie != cudaSuccess) return set_err(TJ_ERR_CUDA, std::string("Lanczos graph: ") + cudaGetErrorString(ie));
   struct ExecGuard {
     cudaGraphExec_t e;
-    ~ExecGuard() { cudaGraphExecDestroy(e); }
-  } guard{exec};
+    cudaStream_t s, side;
+    ~ExecGuard() {
+      cudaStreamSynchronize(s);   // an iteration launched ahead may still run
+      if (side) cudaStreamSynchronize(side);
+      cudaGraphExecDestroy(e);
+    }
+  } guard{exec, st, side};
+  // A short vector's next iteration is launched before this one's scalars are
+  // known, and the Ritz value (one block) is found beside it on a second
+  // stream (2x16 ladder m = 256: 77 us an iteration
+  // with both in line, 57 so).  The iteration launched past the last is dropped as
+  // above, and its error flags with it: the flags are those published with the
+  // scalars.  A long vector's iteration costs more than all those gaps.
+  int flags = 0;
+  int launched = 1;   // the step after the last one launched
   while (last < LOOP_IN) {
-    CK(cudaGraphLaunch(exec, st));
-    CK(cudaStreamSynchronize(st));
+    for (; launched <= last + (is_short ? 1 : 0) && launched < LOOP_IN; ++launched) {
+      CK(cudaGraphLaunch(exec, st));
+      CK(cudaEventRecord(ctx->ev[launched & 1], st));
+      if (!is_short) continue;
+      CK(cudaStreamWaitEvent(side, ctx->ev[launched & 1], 0));
+      launch_lz_publish_short(S, launched, ctx->pinned, side);
+      CK(cudaEventRecord(ctx->ev[2 + (launched & 1)], side));
+    }
+    CK(cudaEventSynchronize(ctx->ev[(is_short ? 2 : 0) + (last & 1)]));
     ++ctx->n_hpsi;
-    hb = ctx->pinned[0];
-    hl = ctx->pinned[1];
+    const double *seen = ctx->pinned + LZ_HOST * (last % LZ_RING);
+    hb = seen[0];
+    hl = seen[1];
+    flags = (int)seen[2];
     ++last;
     if (!std::isfinite(hb)) return set_err(TJ_ERR_NUMERIC, "Lanczos: non-finite beta");
     if (std::fabs(hb) <= lanzero) {
@@ -718,6 +761,7 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
     }
     ritzmin = hl;
   }
+  if (is_short) CK(cudaStreamWaitEvent(st, ctx->ev[2 + ((launched - 1) & 1)], 0));
   // label 411: dstev('V') and the Ritz vector
   launch_tridiag_min(alpha + 1, beta + 1, last, lam, dz, 1, ctx->stream);
   if ((rc = ctx->vout.reserve(sizeof(double) * (D + 4)))) return rc;
@@ -728,7 +772,7 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   if ((rc = download(ctx, eigvec->data, ctx->vout.d(), D, ctx->stream))) return rc;
   if ((rc = res_keep(ctx, eigvec->data, D, ctx->vout.d(), ctx->stream))) return rc;
   if ((rc = fetch(lam, &hl))) return rc;
-  if ((rc = check_device_flags(ctx))) return rc;
+  if ((rc = report_flags(flags))) return rc;
   energies[0] = hl;
   *iters = last;
   ctx->stats.lanczos_hpsi = ctx->n_hpsi - h0;

@@ -4,8 +4,14 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
+
+#include <cooperative_groups.h>
 
 #include "kernels.cuh"
+#include "sturm.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tjb {
 
@@ -534,26 +540,12 @@ void launch_sum(const double *partials, int nblk, double *res, int sqrt_flag, cu
   sum_kernel<<<1, VT, 0, s>>>(partials, nblk, res, sqrt_flag);
 }
 
-__global__ void lanczos_update_kernel(double *y, const double *x1, const double *x2, const double *a,
-                                      const double *b, int64_t n) {
-  const double av = *a, bv = x2 ? *b : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double v = y[i] - av * x1[i];
-    if (x2) v = v - bv * x2[i];
-    y[i] = v;
-  }
-}
 static int vgrid(int64_t n) {
   int64_t g = (n + VT - 1) / VT;
   if (g > 148 * 16) g = 148 * 16;
   if (g < 1) g = 1;
   return (int)g;
 }
-void launch_lanczos_update(double *y, const double *x1, const double *x2, const double *a, const double *b,
-                           int64_t n, cudaStream_t s) {
-  lanczos_update_kernel<<<vgrid(n), VT, 0, s>>>(y, x1, x2, a, b, n);
-}
-
 __global__ void scale_inv_kernel(double *x, const double *nrm, int64_t n) {
   const double d = *nrm;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -561,49 +553,6 @@ __global__ void scale_inv_kernel(double *x, const double *nrm, int64_t n) {
 }
 void launch_scale_inv(double *x, const double *nrm, int64_t n, cudaStream_t s) {
   scale_inv_kernel<<<vgrid(n), VT, 0, s>>>(x, nrm, n);
-}
-
-// Gram-Schmidt projections: each block keeps its slice of w in registers and
-// streams the k basis vectors past it.
-constexpr int MD_PER = 8;
-__global__ void multi_dot_kernel(const double *__restrict__ V, int64_t ld, int k, const double *__restrict__ w,
-                                 int64_t n, double *partials, int kmax) {
-  __shared__ double sh[VT / 32];
-  const int64_t base = (int64_t)blockIdx.x * VT * MD_PER + threadIdx.x;
-  double wr[MD_PER];
-#pragma unroll
-  for (int i = 0; i < MD_PER; ++i) {
-    const int64_t e = base + (int64_t)i * VT;
-    wr[i] = e < n ? w[e] : 0.0;
-  }
-  for (int j = 0; j < k; ++j) {
-    const double *v = V + (int64_t)j * ld;
-    double s = 0.0;
-#pragma unroll
-    for (int i = 0; i < MD_PER; ++i) {
-      const int64_t e = base + (int64_t)i * VT;
-      if (e < n) s += v[e] * wr[i];
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) partials[(int64_t)blockIdx.x * kmax + j] = s;
-  }
-}
-void launch_multi_dot(const double *V, int64_t ld, int k, const double *w, int64_t n, double *partials, int nblk,
-                      int kmax, cudaStream_t s) {
-  multi_dot_kernel<<<nblk, VT, 0, s>>>(V, ld, k, w, n, partials, kmax);
-}
-
-__global__ void multi_sum_kernel(const double *partials, int nblk, int kmax, const double *uu, double *coef) {
-  __shared__ double sh[VT / 32];
-  const int j = blockIdx.x;
-  double s = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partials[(int64_t)b * kmax + j];
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) coef[j] = uu ? s / uu[j] : s;
-}
-void launch_multi_sum(const double *partials, int nblk, int k, int kmax, const double *uu, double *coef,
-                      cudaStream_t s) {
-  if (k > 0) multi_sum_kernel<<<k, VT, 0, s>>>(partials, nblk, kmax, uu, coef);
 }
 
 __global__ void combine_kernel(const double *__restrict__ V, int64_t ld, int k, const double *__restrict__ coef,
@@ -620,20 +569,6 @@ __global__ void combine_kernel(const double *__restrict__ V, int64_t ld, int k, 
 void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, int assign,
                     cudaStream_t s) {
   combine_kernel<<<vgrid(n), VT, 0, s>>>(V, ld, k, coef, w, n, assign);
-}
-
-// Number of eigenvalues of the tridiagonal (a, b2 = b*b) below x (Sturm count).
-__device__ __forceinline__ int sturm_count(const double *a, const double *b2, int n, double x) {
-  const double tiny = 1e-300;
-  int cnt = 0;
-  double q = a[0] - x;
-  if (q < 0) ++cnt;
-  for (int i = 1; i < n; ++i) {
-    if (fabs(q) < tiny) q = -tiny;
-    q = (a[i] - x) - b2[i - 1] / q;
-    if (q < 0) ++cnt;
-  }
-  return cnt;
 }
 
 // Ordered integer image of a double: monotone in the value, with +0 and -0
@@ -664,6 +599,7 @@ constexpr int TRI_THREADS = 256;   // threads (multisection points) of the tridi
 // the hint wide; the bracket at the end is the same either way.
 __device__ void tridiag_min_bracket(const double *a, const double *b, int n, double hint, double &lo_out,
                                     double &hi_out) {
+  // the matrix scaled to a largest row sum below one, its off-diagonal squared
   __shared__ double sa[128], sb2[128], slo[TRI_THREADS / 32], shi[TRI_THREADS / 32];
   __shared__ unsigned sv[TRI_THREADS / 32], su[TRI_THREADS / 32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -671,8 +607,6 @@ __device__ void tridiag_min_bracket(const double *a, const double *b, int n, dou
   // and max of a[i] -+ (|b[i-1]| + |b[i]|), exact in any order)
   double lo = INFINITY, hi = -INFINITY;
   for (int i = t; i < n; i += blockDim.x) {
-    sa[i] = a[i];
-    sb2[i] = i < n - 1 ? b[i] * b[i] : 0.0;
     const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i < n - 1 ? fabs(b[i]) : 0.0);
     lo = fmin(lo, a[i] - r);
     hi = fmax(hi, a[i] + r);
@@ -693,6 +627,13 @@ __device__ void tridiag_min_bracket(const double *a, const double *b, int n, dou
     lo = fmin(lo, slo[q]);
     hi = fmax(hi, shi[q]);
   }
+  const double sc = tridiag_scale(fmax(fabs(lo), fabs(hi)));
+  for (int i = t; i < n; i += blockDim.x) {
+    const double bs = i < n - 1 ? b[i] * sc : 0.0;
+    sa[i] = a[i] * sc;
+    sb2[i] = bs * bs;
+  }
+  __syncthreads();
   // invariant: count(lo) = 0 < count(hi) (Gershgorin bounds)
   // images lie in (-2^63, 2^63), so their distance can exceed the int64
   // range: spans and offsets are taken modulo 2^64, where they are exact
@@ -720,7 +661,7 @@ __device__ void tridiag_min_bracket(const double *a, const double *b, int n, dou
     auto pt = [&](int j) { return geo ? hint_point(j, klo) : point(j, klo, khi); };
     const int64_t kx = pt(t);
     const bool valid = kx > klo && kx < khi;
-    const bool up = valid && sturm_count(sa, sb2, n, val_of(kx)) >= 1;
+    const bool up = valid && sturm1(sa, sb2, n, val_of(kx) * sc) >= 1;
     const unsigned vm = __ballot_sync(0xffffffffu, valid), um = __ballot_sync(0xffffffffu, up);
     if (lane == 0) {
       sv[w] = vm;
@@ -762,36 +703,36 @@ __device__ void tridiag_min_body(const double *a, const double *b, int n, double
   int piv[128];
   double scale = fabs(hi) + fabs(lo) + 1.0;
   for (int i = 0; i < n; ++i) x[i] = 1.0;
-  for (int iter = 0; iter < 3; ++iter) {
-    for (int i = 0; i < n; ++i) {
-      dd[i] = a[i] - l;
-      du[i] = i < n - 1 ? b[i] : 0.0;
-      dl[i] = i < n - 1 ? b[i] : 0.0;
-      du2[i] = 0.0;
-    }
-    // LU with partial pivoting (dgttrf-like)
-    for (int i = 0; i < n - 1; ++i) {
-      if (fabs(dd[i]) >= fabs(dl[i])) {
-        piv[i] = 0;
-        if (dd[i] == 0.0) dd[i] = 1e-300 * scale + 1e-300;
-        const double f = dl[i] / dd[i];
-        dl[i] = f;
-        dd[i + 1] -= f * du[i];
-      } else {
-        piv[i] = 1;
-        const double f = dd[i] / dl[i];
-        dd[i] = dl[i];
-        dl[i] = f;
-        const double t = du[i];
-        du[i] = dd[i + 1];
-        dd[i + 1] = t - f * dd[i + 1];
-        if (i < n - 2) {
-          du2[i] = du[i + 1];
-          du[i + 1] = -f * du[i + 1];
-        }
+  for (int i = 0; i < n; ++i) {
+    dd[i] = a[i] - l;
+    du[i] = i < n - 1 ? b[i] : 0.0;
+    dl[i] = i < n - 1 ? b[i] : 0.0;
+    du2[i] = 0.0;
+  }
+  // LU with partial pivoting (dgttrf-like)
+  for (int i = 0; i < n - 1; ++i) {
+    if (fabs(dd[i]) >= fabs(dl[i])) {
+      piv[i] = 0;
+      if (dd[i] == 0.0) dd[i] = 1e-300 * scale + 1e-300;
+      const double f = dl[i] / dd[i];
+      dl[i] = f;
+      dd[i + 1] -= f * du[i];
+    } else {
+      piv[i] = 1;
+      const double f = dd[i] / dl[i];
+      dd[i] = dl[i];
+      dl[i] = f;
+      const double t = du[i];
+      du[i] = dd[i + 1];
+      dd[i + 1] = t - f * dd[i + 1];
+      if (i < n - 2) {
+        du2[i] = du[i + 1];
+        du[i + 1] = -f * du[i + 1];
       }
     }
-    if (dd[n - 1] == 0.0) dd[n - 1] = 1e-16 * scale;
+  }
+  if (dd[n - 1] == 0.0) dd[n - 1] = 1e-16 * scale;
+  for (int iter = 0; iter < 3; ++iter) {
     // solve L U y = x
     for (int i = 0; i < n - 1; ++i) {
       if (piv[i] == 0) {
@@ -860,93 +801,148 @@ __device__ void lz_grid_sum(double s, double *partials, int *cnt, double *res, i
   }
 }
 
-// vec(L+1) = H vec(L) - alpha(L) vec(L) - beta(L-1) vec(L-1); beta(L) = |vec(L+1)|
-__global__ void lz_update_norm_kernel(LzRef dst, const double *__restrict__ src, LzRef x1, LzRef x2, double *S,
-                                      const int *it, int64_t n, double *partials, int *cnt) {
-  __shared__ double sh[VT / 32];
-  const int L = *it;
-  const double av = S[L], bv = L >= 2 ? S[128 + L - 1] : 0.0;
-  double *__restrict__ y = lz_ptr(dst);
-  const double *__restrict__ p1 = lz_ptr(x1);
-  const double *__restrict__ p2 = L >= 2 ? lz_ptr(x2) : nullptr;
-  double s = 0.0;
-#pragma unroll 4
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double v = src[i] - av * p1[i];
-    if (p2) v = v - bv * p2[i];
-    y[i] = v;
-    s += v * v;
-  }
-  s = block_sum(s, sh);
-  lz_grid_sum(s, partials, cnt, S + 128 + L, 1, sh);
+// A long vector is cut into lz_slices equal slices of lz_slice(n) entries (the
+// last may be short), one per block and two blocks per SM, so that every SM
+// reads the same share of the vectors; at most LZ_SLICE entries, 64 KB.
+constexpr int LZ_SLICE = 8192, LZ_THREADS = 512, LZ_PARTS = 4;
+constexpr int LZ_KMAX = 128;
+int lz_slices(int64_t n) {
+  const int64_t w = 148 * 2;
+  return (int)(w * std::max<int64_t>(1, (n + w * LZ_SLICE - 1) / (w * LZ_SLICE)));
+}
+static int lz_slice(int64_t n) {
+  const int s = lz_slices(n);
+  return (int)((n + s - 1) / s + 1) / 2 * 2;
 }
 
-// Projections of w / beta(L) on vec(1..L), with w scaled in place: each block
-// keeps its slice of w in registers and streams the L vectors past it (the
-// kernel is bound by those reads: L vectors of n doubles).  Five resident
-// blocks per SM put the grid (one block per VT * MD_PER elements: 685 for
-// 1.4M) in one wave on 148 SMs.
-__global__ void __launch_bounds__(VT, 5) lz_multi_dot_kernel(const double *__restrict__ V, int64_t ld, const int *it, LzRef wr_, int64_t n,
-                                    const double *S, double *partials, int kmax) {
-  __shared__ double sh[VT / 32];
-  const int L = *it;
+// w = src - alpha(L) vec(L) - beta(L-1) vec(L-1), its square sum and its
+// projections on vec(1..L): each block keeps its slice of w in shared memory
+// and its warps take the L vectors' slices in quarters, so that no barrier
+// stands between the reads (the kernel is bound by those: L vectors of n
+// doubles).  1.4M entries, 23 vectors on average: 12 us for w and 54 for the
+// projections when each was a kernel, the latter with a block-wide sum per
+// vector; 54 for both now, 39 for the vectors alone at the copy bandwidth.
+// Vectors have an even stride; what lies past n is masked.
+__global__ void __launch_bounds__(LZ_THREADS, 2)
+    lz_update_dots_kernel(const double *__restrict__ V, int64_t ld, const int *it, LzRef wr_,
+                          const double *__restrict__ src, int64_t n, int per, const double *S, double *partials,
+                          int kmax) {
+  extern __shared__ double2 lz_w[];
+  __shared__ double hp[LZ_KMAX][LZ_PARTS], sh[LZ_THREADS / 32];
+  const int L = *it, tid = threadIdx.x, lane = tid & 31;
   const int k = min(L, kmax);
-  const double d = S[128 + L];
-  double *__restrict__ w = lz_ptr(wr_);
-  const int64_t base = (int64_t)blockIdx.x * VT * MD_PER + threadIdx.x;
-  double wr[MD_PER];
-#pragma unroll
-  for (int i = 0; i < MD_PER; ++i) {
-    const int64_t e = base + (int64_t)i * VT;
-    wr[i] = 0.0;
-    if (e < n) {
-      wr[i] = w[e] / d;
-      w[e] = wr[i];
+  const double av = S[L], bv = L >= 2 ? S[128 + L - 1] : 0.0;
+  const int64_t r0 = min(n, (int64_t)blockIdx.x * per);
+  const int nr = (int)min((int64_t)per, n - r0), np = (nr + 1) / 2;
+  double2 *__restrict__ w = reinterpret_cast<double2 *>(lz_ptr(wr_) + r0);
+  const double2 *__restrict__ y = reinterpret_cast<const double2 *>(src + r0);
+  const double2 *__restrict__ p1 = reinterpret_cast<const double2 *>(V + (int64_t)(L - 1) * ld + r0);
+  const double2 *__restrict__ p2 = L >= 2 ? p1 - ld / 2 : nullptr;
+  double q = 0.0;
+#pragma unroll 2
+  for (int i = tid; i < np; i += LZ_THREADS) {
+    const double2 a = y[i], b = p1[i];
+    double2 x = make_double2(a.x - av * b.x, a.y - av * b.y);
+    if (p2) {
+      const double2 c = p2[i];
+      x.x = x.x - bv * c.x;
+      x.y = x.y - bv * c.y;
     }
+    if (2 * i + 1 >= nr) x.y = 0.0;
+    w[i] = x;
+    lz_w[i] = x;
+    q += x.x * x.x;
+    q += x.y * x.y;
   }
-  for (int j = 0; j < k; ++j) {
-    const double *v = V + (int64_t)j * ld;
+  q = block_sum(q, sh);
+  if (tid == 0) partials[(int64_t)blockIdx.x * (kmax + 1) + kmax] = q;
+  const int pp = (np + LZ_PARTS - 1) / LZ_PARTS;
+  for (int u = tid >> 5; u < k * LZ_PARTS; u += LZ_THREADS / 32) {
+    const int j = u / LZ_PARTS, i0 = u % LZ_PARTS * pp, i1 = min(np, i0 + pp);
+    const double2 *__restrict__ v = reinterpret_cast<const double2 *>(V + (int64_t)j * ld + r0);
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 8
+    for (int i = i0 + lane; i < i1; i += 32) {
+      const double2 x = v[i], y = lz_w[i];
+      s0 += x.x * y.x;
+      s1 += (2 * i + 1 < nr ? x.y : 0.0) * y.y;
+    }
+    s0 += s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_down_sync(0xffffffffu, s0, o);
+    if (lane == 0) hp[j][u % LZ_PARTS] = s0;
+  }
+  __syncthreads();
+  for (int j = tid; j < k; j += LZ_THREADS) {
     double s = 0.0;
 #pragma unroll
-    for (int i = 0; i < MD_PER; ++i) {
-      const int64_t e = base + (int64_t)i * VT;
-      if (e < n) s += v[e] * wr[i];
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) partials[(int64_t)blockIdx.x * kmax + j] = s;
+    for (int q = 0; q < LZ_PARTS; ++q) s += hp[j][q];
+    partials[(int64_t)blockIdx.x * (kmax + 1) + j] = s;
   }
 }
 
-// coef(j) = (sum of the block projections) / uu(j), one block per vector
-__global__ void lz_multi_sum_kernel(const double *partials, int nblk, int kmax, const double *uu, double *coef,
-                                    const int *it) {
+// beta(L) = |w| and coef(j) = (w . vec(j)) / beta(L) / uu(j), one block per vector
+__global__ void lz_coef_kernel(const double *partials, int nblk, int kmax, const double *uu, double *coef, double *S,
+                               const int *it) {
   __shared__ double sh[VT / 32];
-  const int j = blockIdx.x;
-  if (j >= *it) return;
-  double s = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partials[(int64_t)b * kmax + j];
+  const int j = blockIdx.x, L = *it;
+  if (j >= L) return;
+  double s = 0.0, q = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    s += partials[(int64_t)b * (kmax + 1) + j];
+    q += partials[(int64_t)b * (kmax + 1) + kmax];
+  }
   s = block_sum(s, sh);
-  if (threadIdx.x == 0) coef[j] = s / uu[j];
+  q = block_sum(q, sh);
+  if (threadIdx.x != 0) return;
+  const double beta = sqrt(q);
+  coef[j] = s / beta / uu[j];
+  if (j == 0) S[128 + L] = beta;
 }
 
-// w -= sum_j coef(j) vec(j); S[513] = |w|
-constexpr int LZ_KMAX = 128;
-__global__ void lz_combine_norm_kernel(const double *__restrict__ V, int64_t ld, const int *it,
-                                       const double *__restrict__ coef, LzRef wr_, int64_t n, double *S,
-                                       double *partials, int *cnt) {
+// w = w / beta(L) - sum_j coef(j) vec(j); S[513] = |w|.  Bound by the reads of
+// the vectors again (1.4M entries, 23 vectors: 54 us with one load in flight a
+// thread, 50 with eight of 16 bytes).
+__global__ void __launch_bounds__(LZ_THREADS, 2)
+    lz_combine_norm_kernel(const double *__restrict__ V, int64_t ld, const int *it, const double *__restrict__ coef,
+                           LzRef wr_, int64_t n, int per, double *S, double *partials, int *cnt) {
   __shared__ double c[LZ_KMAX];
-  __shared__ double sh[VT / 32];
+  __shared__ double sh[32];
   const int k = min(*it, LZ_KMAX);
-  double *__restrict__ w = lz_ptr(wr_);
   for (int j = threadIdx.x; j < k; j += blockDim.x) c[j] = coef[j];
   __syncthreads();
+  const int64_t r0 = min(n, (int64_t)blockIdx.x * per);
+  const int nr = (int)min((int64_t)per, n - r0), np = (nr + 1) / 2;
+  double2 *__restrict__ w = reinterpret_cast<double2 *>(lz_ptr(wr_) + r0);
+  const double2 *__restrict__ v0 = reinterpret_cast<const double2 *>(V + r0);
+  const int64_t ld2 = ld / 2;
+  const double beta = S[128 + *it];
   double s = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (int j = 0; j < k; ++j) t = t + c[j] * V[(int64_t)j * ld + i];
-    const double v = w[i] - t;
-    w[i] = v;
-    s += v * v;
+  for (int i = threadIdx.x; i < np; i += LZ_THREADS) {
+    double2 t = make_double2(0.0, 0.0), y = w[i];
+    const double2 *x = v0 + i;
+    int j = 0;
+    for (; j + 8 <= k; j += 8, x += 8 * ld2) {   // eight loads in flight
+      double2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = x[u * ld2];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        t.x = t.x + c[j + u] * v[u].x;
+        t.y = t.y + c[j + u] * v[u].y;
+      }
+    }
+#pragma unroll 4
+    for (; j < k; ++j, x += ld2) {
+      const double2 v = *x;
+      t.x = t.x + c[j] * v.x;
+      t.y = t.y + c[j] * v.y;
+    }
+    y.x = y.x / beta - t.x;
+    y.y = 2 * i + 1 < nr ? y.y / beta - t.y : 0.0;
+    w[i] = y;
+    s += y.x * y.x;
+    s += y.y * y.y;
   }
   s = block_sum(s, sh);
   lz_grid_sum(s, partials, cnt, S + 513, 1, sh);
@@ -985,35 +981,224 @@ __global__ void lz_dot_kernel(LzRef xr, const double *__restrict__ y, int64_t n,
   lz_grid_sum(s, partials, cnt, S + 1 + L, 0, sh);
 }
 
-// The Ritz value of T(L+1); beta(L) and the Ritz value to page-locked host
-// memory; the step advances.
-__global__ void lz_tridiag_publish_kernel(double *S, int *it, double *host) {
-  const int L = *it;
+// The Ritz value of T(L+1); beta(L), the Ritz value and the split-precision
+// kernels' error word to step L's place of the ring in page-locked host memory.
+// By one block.
+__device__ void lz_publish(double *S, int L, double flags, double *host) {
   double lo, hi;
   // from the second step on, S[512] holds the Ritz value of the step before
   tridiag_min_bracket(S + 1, S + 129, L + 1, L >= 2 ? S[512] : __longlong_as_double(0x7FF8000000000000LL), lo, hi);
   if (threadIdx.x != 0) return;
   S[512] = 0.5 * (lo + hi);
+  host += LZ_HOST * (L % LZ_RING);
   host[0] = S[128 + L];
   host[1] = S[512];
+  host[2] = flags;
   __threadfence_system();
-  *it = L + 1;
+}
+__global__ void lz_tridiag_publish_kernel(double *S, int *it, const int *err, double *host) {
+  const int L = *it;
+  lz_publish(S, L, err ? (double)*err : 0.0, host);
+  if (threadIdx.x == 0) *it = L + 1;
+}
+// the same of a given step, beside the next one's kernels
+__global__ void lz_publish_short_kernel(double *S, int L, double *host) {
+  lz_publish(S, L, S[LZ_FLAGS + L % LZ_RING], host);
+}
+
+// ---- the same steps for a short vector, by one thread-block cluster: the
+// kernels above need a launch or two for each sum over the vector, and at the
+// sizes of a ladder each of them is all latency (2x16 ladder m = 256, 23,140
+// entries, 25 vectors on average: 42 us for recurrence, projections,
+// combination and scaling as five kernels, 21 now; alpha 5).  CTA c of CL holds
+// entries [c per, (c + 1) per) of the new vector in shared memory; sums meet
+// through distributed shared memory and are added in rank order by everyone.
+constexpr int LZC_THREADS = 512;
+constexpr int LZC_MAX = 4096;   // entries of a CTA
+
+// The sum over the cluster of x, one value per thread, in every thread; slot
+// is used by no other sum of the kernel, red holds LZC_THREADS / 32 doubles.
+template <int CL>
+__device__ __forceinline__ double lz_cluster_sum(cg::cluster_group &cl, double x, double *slot, double *red) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  __syncthreads();
+  if (lane == 0) red[threadIdx.x >> 5] = x;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+  if (threadIdx.x == 0) *slot = s;
+  cl.sync();
+  double p = lane < CL ? *cl.map_shared_rank(slot, lane < CL ? lane : 0) : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+  return p;
+}
+
+// vec(L+1) from H vec(L) in src: recurrence, beta(L), Gram-Schmidt against
+// vec(1..L), normalisation; also to x, with uu(L+1).
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(LZC_THREADS, 1)
+    lz_step_cluster_kernel(double *V, int64_t ld, const int *it, const double *__restrict__ src, double *__restrict__ x,
+                           int64_t n, double *S) {
+  __shared__ double w[LZC_MAX], hp[LZ_KMAX], cf[LZ_KMAX], slot[4], red[LZC_THREADS / 32];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int L = *it, k = min(L, LZ_KMAX);
+  const int per = (int)((n + CL - 1) / CL);
+  const int64_t r0 = min(n, (int64_t)rank * per);
+  const int nr = (int)(min(n, r0 + per) - r0);
+  const double av = S[L], bv = L >= 2 ? S[128 + L - 1] : 0.0;
+  const double *p1 = V + (int64_t)(L - 1) * ld + r0, *p2 = L >= 2 ? p1 - ld : nullptr;
+  double *out = V + (int64_t)L * ld + r0;
+  double s = 0.0;
+  for (int i = tid; i < nr; i += LZC_THREADS) {
+    double v = src[r0 + i] - av * p1[i];
+    if (p2) v = v - bv * p2[i];
+    w[i] = v;
+    s += v * v;
+  }
+  const double beta = sqrt(lz_cluster_sum<CL>(cl, s, slot, red));
+  for (int i = tid; i < nr; i += LZC_THREADS) w[i] = w[i] / beta;
+  __syncthreads();
+  // the CTA's parts of the projections, a warp per vector
+  for (int j = warp; j < k; j += LZC_THREADS / 32) {
+    const double *v = V + (int64_t)j * ld + r0;
+    double a = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < nr; i += 32) a += v[i] * w[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) hp[j] = a;
+  }
+  cl.sync();
+  if (tid < k) {
+    double a = 0.0;
+#pragma unroll
+    for (int c = 0; c < CL; ++c) a += cl.map_shared_rank(hp, c)[tid];
+    cf[tid] = a / S[257 + tid];
+  }
+  __syncthreads();
+  s = 0.0;
+  for (int i = tid; i < nr; i += LZC_THREADS) {
+    double t = 0.0;
+    const double *v = V + r0 + i;
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) t = t + cf[j] * v[(int64_t)j * ld];
+    const double y = w[i] - t;
+    w[i] = y;
+    s += y * y;
+  }
+  const double nrm = sqrt(lz_cluster_sum<CL>(cl, s, slot + 1, red));
+  s = 0.0;
+  for (int i = tid; i < nr; i += LZC_THREADS) {
+    const double y = w[i] / nrm;
+    out[i] = y;
+    x[r0 + i] = y;
+    s += y * y;
+  }
+  const double uu = lz_cluster_sum<CL>(cl, s, slot + 2, red);
+  if (rank == 0 && tid == 0) {
+    S[128 + L] = beta;
+    S[513] = nrm;
+    S[257 + L] = uu;
+  }
+  cl.sync();   // no CTA leaves while another may still read its shared memory
+}
+
+// alpha(L+1) = x . y; the error word to S; the step advances
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(LZC_THREADS, 1)
+    lz_dot_cluster_kernel(const double *__restrict__ x, const double *__restrict__ y, int64_t n, double *S, int *it,
+                          const int *err) {
+  __shared__ double slot, red[LZC_THREADS / 32];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  double s = 0.0;
+#pragma unroll 4
+  for (int i = rank * LZC_THREADS + (int)threadIdx.x; i < n; i += CL * LZC_THREADS) s += x[i] * y[i];
+  s = lz_cluster_sum<CL>(cl, s, &slot, red);
+  if (rank == 0 && threadIdx.x == 0) {
+    const int L = *it;
+    S[1 + L] = s;
+    S[LZ_FLAGS + L % LZ_RING] = err ? (double)*err : 0.0;
+    *it = L + 1;
+  }
+  cl.sync();
+}
+
+// 16 CTAs where the device can place such a cluster (a non-portable size),
+// else 8; asked once
+static int lz_cluster_size() {
+  static std::once_flag once;
+  static int size = 8;
+  std::call_once(once, [] {
+    bool ok = true;
+    auto fits = [&](auto kernel, int threads) {
+      ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(16, 1, 1);
+      cfg.blockDim = dim3(threads, 1, 1);
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 16;
+      attr.val.clusterDim.y = 1;
+      attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int m = 0;
+      ok = ok && cudaOccupancyMaxActiveClusters(&m, kernel, &cfg) == cudaSuccess && m >= 1;
+    };
+    fits(lz_step_cluster_kernel<16>, LZC_THREADS);
+    fits(lz_dot_cluster_kernel<16>, LZC_THREADS);
+    if (ok) size = 16;
+    cudaGetLastError();
+  });
+  return size;
+}
+// Whether the cluster kernels take a vector of n entries.  A cluster reads the
+// earlier vectors through its own 16 SMs only, so the grid-wide kernels win
+// where those reads outweigh the launches (an iteration, cluster against
+// grid: 5,628 entries 43 and 68 us, 23,140 57 and 77, 31,915 63 and 78, 45,315
+// 72 and 81, 61,756 96 and 86).
+bool lz_short(int64_t n) { return n <= 49152 && n <= (int64_t)lz_cluster_size() * LZC_MAX; }
+void launch_lz_step_short(double *V, int64_t ld, const int *it, const double *src, double *x, int64_t n, double *S,
+                          cudaStream_t s) {
+  if (lz_cluster_size() == 16) {
+    cudaFuncSetAttribute(lz_step_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    lz_step_cluster_kernel<16><<<16, LZC_THREADS, 0, s>>>(V, ld, it, src, x, n, S);
+  } else {
+    lz_step_cluster_kernel<8><<<8, LZC_THREADS, 0, s>>>(V, ld, it, src, x, n, S);
+  }
+}
+void launch_lz_dot_short(const double *x, const double *y, int64_t n, double *S, int *it, const int *err,
+                         cudaStream_t s) {
+  if (lz_cluster_size() == 16) {
+    cudaFuncSetAttribute(lz_dot_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    lz_dot_cluster_kernel<16><<<16, LZC_THREADS, 0, s>>>(x, y, n, S, it, err);
+  } else {
+    lz_dot_cluster_kernel<8><<<8, LZC_THREADS, 0, s>>>(x, y, n, S, it, err);
+  }
+}
+void launch_lz_publish_short(double *S, int L, double *host, cudaStream_t s) {
+  lz_publish_short_kernel<<<1, TRI_THREADS, 0, s>>>(S, L, host);
 }
 
 // the elementwise kernels with a fused norm run on the grid of a dot product
 // (fewer partials for the last block to add); the Gram-Schmidt combination,
 // which streams L vectors per element, on the wider vector grid
-int lz_blocks(int64_t n) { return std::max(vgrid(n), dot_blocks(n)); }
-void launch_lz_update_norm(LzRef dst, const double *src, LzRef x1, LzRef x2, double *S, const int *it, int64_t n,
-                           double *partials, int *cnt, cudaStream_t s) {
-  lz_update_norm_kernel<<<dot_blocks(n), VT, 0, s>>>(dst, src, x1, x2, S, it, n, partials, cnt);
-}
-void launch_lz_gram_schmidt(const double *V, int64_t ld, const int *it, LzRef w, int64_t n, double *S,
-                            double *mpartials, int mdb, int kmax, const double *uu, double *coef, double *partials,
-                            int *cnt, cudaStream_t s) {
-  lz_multi_dot_kernel<<<mdb, VT, 0, s>>>(V, ld, it, w, n, S, mpartials, kmax);
-  lz_multi_sum_kernel<<<kmax, VT, 0, s>>>(mpartials, mdb, kmax, uu, coef, it);
-  lz_combine_norm_kernel<<<vgrid(n), VT, 0, s>>>(V, ld, it, coef, w, n, S, partials, cnt);
+int lz_blocks(int64_t n) { return std::max(lz_slices(n), dot_blocks(n)); }
+void launch_lz_update_gram_schmidt(const double *V, int64_t ld, const int *it, LzRef w, const double *src, int64_t n,
+                                   double *S, double *mpartials, int kmax, const double *uu, double *coef,
+                                   double *partials, int *cnt, cudaStream_t s) {
+  const int ns = lz_slices(n), per = lz_slice(n);
+  const int bytes = per * (int)sizeof(double);
+  cudaFuncSetAttribute(lz_update_dots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       LZ_SLICE * (int)sizeof(double));
+  lz_update_dots_kernel<<<ns, LZ_THREADS, bytes, s>>>(V, ld, it, w, src, n, per, S, mpartials, kmax);
+  lz_coef_kernel<<<kmax, VT, 0, s>>>(mpartials, ns, kmax, uu, coef, S, it);
+  lz_combine_norm_kernel<<<ns, LZ_THREADS, 0, s>>>(V, ld, it, coef, w, n, per, S, partials, cnt);
 }
 void launch_lz_scale_norm(LzRef w, double *x, int64_t n, double *S, const int *it, double *partials, int *cnt,
                           cudaStream_t s) {
@@ -1023,16 +1208,8 @@ void launch_lz_dot(LzRef x, const double *y, int64_t n, double *S, const int *it
                    cudaStream_t s) {
   lz_dot_kernel<<<dot_blocks(n), VT, 0, s>>>(x, y, n, S, it, partials, cnt);
 }
-void launch_lz_tridiag_publish(double *S, int *it, double *host, cudaStream_t s) {
-  lz_tridiag_publish_kernel<<<1, TRI_THREADS, 0, s>>>(S, it, host);
-}
-
-__global__ void copy_kernel(double *dst, const double *src, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = src[i];
-}
-void launch_copy(double *dst, const double *src, int64_t n, cudaStream_t s) {
-  copy_kernel<<<vgrid(n), VT, 0, s>>>(dst, src, n);
+void launch_lz_tridiag_publish(double *S, int *it, const int *err, double *host, cudaStream_t s) {
+  lz_tridiag_publish_kernel<<<1, TRI_THREADS, 0, s>>>(S, it, err, host);
 }
 
 }  // namespace tjb

@@ -37,25 +37,14 @@ void launch_merge(double *ops, const int64_t *dst, const int64_t *n, const int32
 void launch_dot(const double *x, const double *y, int64_t n, double *partials, int nblk, cudaStream_t s);
 void launch_sum(const double *partials, int nblk, double *res, int sqrt_flag, cudaStream_t s);
 int dot_blocks(int64_t n);
-// y = y - a[ia]*x1 (- b[ib]*x2 if x2)   (a, b device scalars)
-void launch_lanczos_update(double *y, const double *x1, const double *x2, const double *a, const double *b,
-                           int64_t n, cudaStream_t s);
 // x = x / (*nrm)
 void launch_scale_inv(double *x, const double *nrm, int64_t n, cudaStream_t s);
-// Gram-Schmidt: partial dots of w with V[0..k-1] (vectors of stride ld) -> partials[blk*kmax + j]
-void launch_multi_dot(const double *V, int64_t ld, int k, const double *w, int64_t n, double *partials, int nblk,
-                      int kmax, cudaStream_t s);
-// coef[j] = (sum over blocks of partials[:, j]) / uu[j] ; uu == nullptr -> divide by 1
-void launch_multi_sum(const double *partials, int nblk, int k, int kmax, const double *uu, double *coef,
-                      cudaStream_t s);
 // w = w - sum_j coef[j] * V[j]    (or w = sum_j coef[j] V[j] when assign)
 void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, int assign,
                     cudaStream_t s);
 // lowest eigenvalue (and its eigenvector if vec) of the symmetric tridiagonal (a[0..n-1], b[0..n-2])
 void launch_tridiag_min(const double *a, const double *b, int n, double *lam, double *vec, int want_vec,
                         cudaStream_t s);
-// out = sum of a device array of n doubles into res (deterministic)
-void launch_copy(double *dst, const double *src, int64_t n, cudaStream_t s);
 
 // ---- Lanczos iteration with the step L read from device memory (*it) ----
 // A vector chosen when the kernel runs: vec(*it + off) = V + (*it + off - 1) * ld, or `fixed`.
@@ -71,14 +60,14 @@ struct LzRef {
 // a grid-wide sum count their blocks on (the last block resets it); partials:
 // lz_blocks(n) doubles.
 int lz_blocks(int64_t n);
-// dst = src - alpha(L) x1 - beta(L-1) x2 (x2 only for L >= 2); beta(L) = |dst|
-void launch_lz_update_norm(LzRef dst, const double *src, LzRef x1, LzRef x2, double *S, const int *it, int64_t n,
-                           double *partials, int *cnt, cudaStream_t s);
-// w /= beta(L); w -= sum_{j < L} (V_j . w / uu[j]) V_j (classical Gram-Schmidt
-// against the first L vectors); S[513] = |w|.  mpartials: mdb * kmax doubles.
-void launch_lz_gram_schmidt(const double *V, int64_t ld, const int *it, LzRef w, int64_t n, double *S,
-                            double *mpartials, int mdb, int kmax, const double *uu, double *coef, double *partials,
-                            int *cnt, cudaStream_t s);
+// w = src - alpha(L) vec(L) - beta(L-1) vec(L-1) (the last for L >= 2 only);
+// beta(L) = |w|; w /= beta(L); w -= sum_{j < L} (V_j . w / uu[j]) V_j (classical
+// Gram-Schmidt against the first L vectors); S[513] = |w|.  mpartials:
+// lz_slices(n) * (kmax + 1) doubles, kmax <= 128; ld even.
+int lz_slices(int64_t n);
+void launch_lz_update_gram_schmidt(const double *V, int64_t ld, const int *it, LzRef w, const double *src, int64_t n,
+                                   double *S, double *mpartials, int kmax, const double *uu, double *coef,
+                                   double *partials, int *cnt, cudaStream_t s);
 // w /= S[513], copied to x; uu(L + 1) = w . w
 void launch_lz_scale_norm(LzRef w, double *x, int64_t n, double *S, const int *it, double *partials, int *cnt,
                           cudaStream_t s);
@@ -86,7 +75,20 @@ void launch_lz_scale_norm(LzRef w, double *x, int64_t n, double *S, const int *i
 void launch_lz_dot(LzRef x, const double *y, int64_t n, double *S, const int *it, double *partials, int *cnt,
                    cudaStream_t s);
 // S[512] = lowest eigenvalue of the leading (L + 1) x (L + 1) tridiagonal;
-// host[0] = beta(L), host[1] = S[512] (page-locked host memory); then L += 1
-void launch_lz_tridiag_publish(double *S, int *it, double *host, cudaStream_t s);
+// beta(L), S[512] and *err (0 without err) to host + LZ_HOST * (L % LZ_RING)
+// (page-locked host memory); then L += 1
+constexpr int LZ_HOST = 4, LZ_RING = 4;
+void launch_lz_tridiag_publish(double *S, int *it, const int *err, double *host, cudaStream_t s);
+// A short vector's iteration: launch_lz_step_short for
+// update_gram_schmidt and scale_norm; launch_lz_dot_short for dot, which keeps *err in
+// S[LZ_FLAGS + L % LZ_RING] and advances L; launch_lz_publish_short for the
+// rest of tridiag_publish, of step L, on any stream.
+constexpr int LZ_FLAGS = 740;
+bool lz_short(int64_t n);
+void launch_lz_step_short(double *V, int64_t ld, const int *it, const double *src, double *x, int64_t n, double *S,
+                          cudaStream_t s);
+void launch_lz_dot_short(const double *x, const double *y, int64_t n, double *S, int *it, const int *err,
+                         cudaStream_t s);
+void launch_lz_publish_short(double *S, int L, double *host, cudaStream_t s);
 
 }  // namespace tjb
