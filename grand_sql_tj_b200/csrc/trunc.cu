@@ -43,11 +43,14 @@ namespace tjb {
 
 constexpr int EIG_THREADS = 512;
 constexpr int EIG_MAX_N = 4096;
-constexpr int TD_NX = (EIG_MAX_N + EIG_THREADS - 1) / EIG_THREADS;   // rows of a column per thread
 constexpr double EIG_EPS = 2.220446049250313e-16;        // 2^-52
 constexpr double EIG_SAFMIN = 2.2250738585072014e-308;   // smallest normal FP64
 constexpr int ORTH_THREADS = 512;
-constexpr int TD_BIG = 320;       // sectors of at least this many states are reduced by a whole cluster
+// Sectors of at least this many states are reduced by a whole cluster: alone,
+// 191 states take 0.84 ms in one CTA, 192 take 0.56 in a cluster, 261 1.77 and 0.78,
+// 319 2.98 and 1.00; but only seven clusters of 16 run at a time, so the line
+// lies above the break-even of one sector.
+constexpr int TD_BIG = 192;
 
 // Sum of the warps' partial sums r[0..nw-1] by every warp: lane w takes
 // r[w] and a shuffle tree adds them, in the same order in every warp (a
@@ -249,224 +252,455 @@ __device__ __forceinline__ double block_sum1(double x, double *red, int &half) {
 }
 
 // The same reduction of one large sector by the CL CTAs of a thread-block
-// cluster.  Every CTA forms column k itself (the pending update applied; the
-// same arithmetic in the same order, so the same reflector everywhere, and
-// every thread derives beta, tau and the scale from the same sum); CTA c
-// owns the trailing columns j = c (mod CL), applies the pending rank-2 update
-// to them and forms its part of p = A v, one thread per row, or, when the
-// CTA's threads outnumber the rows, one per row in each of G groups that
-// split the owned columns (the reflector is scaled where it is read).  The
-// parts meet through distributed shared memory as a reduce-scatter and a
-// broadcast, both by remote stores: each CTA stores the parts of rows
-// [o ch, (o + 1) ch) into CTA o's shared memory; after the first cluster
-// barrier CTA o sums them in rank order and stores the sums into every
-// CTA's p; after the second, every CTA reads its own copy.  Per step: two
-// cluster barriers (the first also orders the owners' column writes in
-// global memory before they are read) and three CTA barriers (four with
-// column groups).  Column k + 1, complete at the first barrier, is loaded
-// into registers there for the next step.  The owner of column k stores its
-// reflector there only after the first barrier, when no CTA reads the column
-// any more.
+// cluster, in panels of TD_NB reflectors as LAPACK's dsytrd does it: within a
+// panel the trailing block A stays as it was at the panel's start and a step
+// takes the rank-2 terms of the panel's earlier reflectors from the thin
+// matrices V and W,
+//   w = tau (A v - V (W^T v) - W (V^T v)) - (tau / 2) (p.v) v,
+// and A <- A - V W^T - W V^T follows once per panel.  CTA c owns the columns
+// (and the rows of V and W) j = c (mod CL).  As A is symmetric, entry j of A v
+// is the product of owned column j with v, and entry j of the next column is an
+// entry of owned column j.  A step has two exchanges:
+//   1. the owned entries of column k (every CTA gets the whole column);
+//   2. the CTA's parts of W^T a, V^T a and a.(A a), a the column below row
+//      k + 1, and from the owner of column k + 1 its rows of V, W and A a, from
+//      which every CTA finds that row's new w for itself.
+// The reflector's scale is found by one warp while the others multiply, and
+// enters the sums where they are read.
+// A step is a chain of latencies (8 cycles an FP64 operation, 38 a level of a
+// shuffle sum, 44 a CTA barrier; 48 doubles to each of 16 CTAs under a cluster
+// barrier 2100, counted by the receiver's mbarrier 1380) and, with 16 warps, of
+// instructions: so the exchanges are st.async, whole warps to consecutive
+// places, and V, W, d, e and tau go to global memory at the panel's end only.
+// The columns stay where they are between the panels' ends: as many of the
+// last ones as fit live in the CTA's shared memory from the start, all of them
+// from the first panel at which they fit; the others stream from L2.
+// n = 857 on 16 CTAs: 8.6 us a step (7.3 ms) with the block read, updated and
+// written in each and parts of A v exchanged under cluster barriers, 4.8 (4.1 ms)
+// so; n = 320: 4.2 and 3.0.
+constexpr int TD_NB = 16;              // reflectors of a panel
+constexpr int TD_LD = 2 * TD_NB + 2;   // row of V and W in shared memory: V, W, pad
+constexpr int TD_PT = 3 * TD_NB;       // a CTA's parts: W^T a, V^T a, a.(A a) by warp
+constexpr long long TD_WAIT = 4000000000LL;   // cycles until a wait for the other CTAs' stores gives up
+constexpr int TD_PL = TD_PT + 1;       // their stride: odd, so that the CTAs' parts lie in different banks
+
+// Doubles of shared memory besides the resident columns.
+__host__ __device__ constexpr int td_coop_doubles(int n, int cl) {
+  const int own = (n + cl - 1) / cl;
+  return own * TD_LD + cl * (own | 1) + 2 * own + (cl + 1) * TD_PL + 2 * TD_LD + 3 * TD_NB + 8;
+}
+
+// acc[c] = column c . a, this lane's rows being i0, i0 + 32, ... below n; a is
+// kept by owner (row i at (i mod CL) lc + i / CL).  dw and dv are summed over the
+// warp with them if more.
+template <int NC, int XS>
+__device__ __forceinline__ void td_dots(const double *const (&p)[4], const double *x, int i0, int n, double (&acc)[4],
+                                        bool more, double &dw, double &dv) {
+#pragma unroll 4
+  for (int i = i0; i < n; i += 32, x += XS) {
+    const double a = *x;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] += a * p[c][i];
+  }
+  if (more) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+      dw += __shfl_xor_sync(0xffffffffu, dw, o);
+      dv += __shfl_xor_sync(0xffffffffu, dv, o);
+    }
+  } else {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+  }
+}
+
+__device__ __forceinline__ uint32_t td_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// the shared-memory address of CTA r's copy of this CTA's place a
+__device__ __forceinline__ uint32_t td_remote(uint32_t a, int r) {
+  uint32_t o;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
+  return o;
+}
+// v to another CTA's shared memory, counted there on the mbarrier bar
+__device__ __forceinline__ void td_send(uint32_t dst, double v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void td_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase of the given parity; false if it does not come (TD_WAIT).
+__device__ __forceinline__ bool td_wait(uint32_t bar, uint32_t parity) {
+  const long long c0 = clock64();
+  do {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  } while (clock64() - c0 < TD_WAIT);
+  return false;
+}
+__device__ __forceinline__ void td_dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 template <int CL>
 __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aall, const int64_t *off,
                              const int *dims, const int64_t *eoff, double *dall, double *eall, double *tauall,
-                             double *info, double *dsall, double *e2all, double *sm, int64_t smem_doubles, double *red2,
-                             double *pvs) {
-  const int n = dims[s], tid = threadIdx.x, nt = blockDim.x;
-  double *A = Aall + off[s];
+                             double *Wall, double *info, double *dsall, double *e2all, double *sm, int64_t smem_doubles,
+                             double *red, uint64_t *mbar, int *status) {
+  constexpr int NB = TD_NB, NW = EIG_THREADS / 32, MW = NW - 1;   // MW warps multiply, the last finds the scale
+  static_assert(NB == 16 && NW == 16 && CL <= NW, "the warps' shares below");
+  const int n = dims[s], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *A = Aall + off[s], *Wg = Wall + NB * eoff[s];   // Wg: W, column-major
   double *d = dall + eoff[s], *e = eall + eoff[s], *tau = tauall + eoff[s];
-  // vp, wp, v: n each; cp: the bin of parts of A v sent to this CTA (CL x
-  // ceil(m / CL) <= 2n); pp: p = tau A v, n
-  // gp: the column groups' parts of A v when a CTA's threads outnumber the
-  // trailing rows (G groups, G * m <= nt entries); sl: the CTA's slice of the
-  // trailing block, the rest of the shared memory
-  double *vp = sm, *wp = vp + n, *v = wp + n, *cp = v + n, *pp = cp + 2 * n, *gp = pp + n, *sl = gp + nt;
-  // From step kres on, when the trailing block has mres = n - 1 - kres rows,
-  // each CTA's owned columns (ceil(mres / CL) of them at most) live in its
-  // slice: owned column j >= jr0(c), row i >= kres + 1 at
-  // sl[(j - jr0(c)) / CL * mres + i - kres - 1].  Step kres reads them from
-  // global memory and writes them there; later steps touch only the slice,
-  // and the other CTAs read the next column from its owner's slice.
-  const int64_t cap = smem_doubles - (6 * (int64_t)n + nt);
-  int mres = 0;
-  if (cap > 0) {
-    mres = min(n - 1, (int)sqrt((double)cap * CL));
-    while (mres > 0 && (int64_t)((mres + CL - 1) / CL) * mres > cap) --mres;
+  const int own = (n + CL - 1) / CL, lc = own | 1;        // an odd stride: no bank conflicts across owners
+  const int nq = rank < n ? (n - 1 - rank) / CL + 1 : 0;  // owned columns rank + q CL
+  auto own_from = [&](int i) { return i <= rank ? 0 : (i - rank + CL - 1) / CL; };  // first q with rank + q CL >= i
+  double *vw = sm;                  // owned rows of V and W
+  double *col = vw + own * TD_LD;   // column k: row i at (i % CL) lc + i / CL
+  double *me = col + rank * lc;     // its owned entries
+  double *ys = col + CL * lc;       // owned entries of A a (rows below k + 1 only)
+  double *rk = ys + own;            // owned entries of row k + 1 of A
+  double *part = rk + own;          // by CTA: its parts (TD_PT)
+  double *stg = part + CL * TD_PL;  // the parts to send
+  double *rb = stg + TD_PL;         // row k of V (NB), of W (NB), entries k of ys and rk
+  double *cs = rb + TD_LD;          // W^T v, V^T v, a.(A a)
+  double *de = cs + TD_LD;          // the panel's d, e, tau (NB each)
+  double *sc = de + 3 * NB;         // scale and tau of the step
+  double *sl = sc + 8;              // resident columns
+  const int64_t cap = smem_doubles - td_coop_doubles(n, CL);
+  // owned columns q >= qr are resident: row i of column q at sl[(q - qr) st + i - r0]
+  int qr = nq - (int)min((int64_t)nq, max((int64_t)0, cap / n)), st = n, r0 = 0;
+  auto res = [&](int q) -> double * { return sl + (int64_t)(q - qr) * st - r0; };
+  auto glo = [&](int q) -> double * { return A + (int64_t)(rank + q * CL) * n; };
+  for (int q = qr + warp; q < nq; q += NW)
+    for (int i = lane; i < n; i += 32) res(q)[i] = glo(q)[i];
+  // The exchanges: mbar[0] counts the bytes of column k, mbar[1] those of the
+  // parts, one phase a step.  No buffer is doubled: a CTA sends its entries of
+  // the next column once it has every CTA's parts, which each sends after its
+  // last read of this column, and its next parts once it has every CTA's
+  // entries, sent after the last read of the parts before.
+  const uint32_t bar0 = td_smem(mbar), bar1 = td_smem(mbar + 1);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const int kres = n - 1 - mres, kr1 = kres + 1;
-  auto jr0 = [&](int c) { return kr1 + ((c - kr1) % CL + CL) % CL; };
-  const int myr0 = jr0(rank);
-  int half = 0;
-  bool pending = false;
-  // rows k + tid + c nt of column k, loaded during step k - 1 (n <= TD_NX nt)
-  double nx[TD_NX];
-  for (int k = 0; k + 1 < n; ++k) {
-    const int k1 = k + 1, m = n - k1;
-    const bool owner = (k % CL) == rank;
-    double *colk = A + (int64_t)k * n;
-    double ss = 0.0;
+  bool late = false;   // a wait has given up: the rest runs through without waiting
+  int p = 0;   // the panel's first column
+  // the panel's V (below each reflector's first row), d, e and tau to global memory
+  auto flush = [&](int cols) {
+    const int qp = own_from(p + 1);
+    for (int x = tid; x < (nq - qp) * NB; x += EIG_THREADS) {
+      const int q = qp + x / NB, l = x % NB, i = rank + q * CL;
+      if (l < cols && i > p + l) A[(int64_t)(p + l) * n + i] = vw[q * TD_LD + l];
+    }
+    if (rank == 0 && tid < cols) {
+      d[p + tid] = de[tid];
+      e[p + tid] = de[NB + tid];
+      tau[p + tid] = de[2 * NB + tid];
+    }
+  };
+  cl.sync();
+  for (int k = 0;; ++k) {
+    // ---- v and w of step k - 1 (its panel column L), then the owned entries of column k
+    const int q0 = own_from(k);
+    const int grp = tid >> 3, h = tid & 7;
+    bool fresh = k == p;   // column k is that of A itself
+    if (!fresh) {
+      const int L = k - 1 - p;
+      const double scl = sc[0], t = sc[1];
+      {
+        const int dn = tid >> 4, r = tid & 15;
+        double x = r < CL && (dn & 15) < L ? part[r * TD_PL + dn] : 0.0, y = 0.0;
+        if (warp == MW) {
 #pragma unroll
-    for (int c = 0; c < TD_NX; ++c) {
-      const int i = k + tid + c * nt;
-      if (i < n) {
-        double a = k == 0 ? colk[i] : nx[c];
-        if (pending) a -= vp[i] * wp[k] + wp[i] * vp[k];
-        v[i] = a;
-        if (i > k1) ss += a * a;
+          for (int u = 0; u < CL / 2; ++u) y += part[(2 * u + (lane >> 4)) * TD_PL + 2 * NB + (lane & 15)];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+          x += __shfl_xor_sync(0xffffffffu, x, o);
+          y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        if (r == 0) cs[dn] = x * scl + ((dn & 15) < L ? rb[dn ^ 16] : 0.0);
+        if (warp == MW) {
+          y += __shfl_xor_sync(0xffffffffu, y, 16);
+          if (lane == 0) cs[2 * NB] = y;
+        }
       }
-    }
-    const double sigma2 = block_sum1(ss, red2, half);   // also the barrier after v
-    const double alpha = v[k1];
-    double beta = alpha, t = 0.0, scl = 0.0;
-    if (sigma2 > 0.0) {
-      const double nr = sqrt(alpha * alpha + sigma2);
-      beta = alpha >= 0.0 ? -nr : nr;
-      t = (beta - alpha) / beta;
-      scl = 1.0 / (alpha - beta);
-    }
-    if (owner && tid == 0) {
-      d[k] = v[k];
-      e[k] = beta;
-      tau[k] = t;
-    }
-    // the scaled reflector: 1 at k1, v[i] * scl below
-    auto rv = [&](int i) { return i == k1 ? 1.0 : v[i] * scl; };
-    // owned trailing columns j0, j0 + CL, ... (mloc of them): rows r, r + R,
-    // ... by the R threads of each of G column groups, group g taking the
-    // owned columns q = g, g + G, ...
-    const int j0 = k1 + ((rank - k1) % CL + CL) % CL;
-    const int mloc = j0 < n ? (n - 1 - j0) / CL + 1 : 0;
-    const int R = min((m + 31) & ~31, nt), G = nt / R;
-    const int g = tid / R, r = tid - g * R;
-    // the parts of A v go to the CTA that sums their rows: rows [o ch, (o + 1)
-    // ch) to CTA o, whose bin holds CL rows of ch slots (by sender)
-    const int ch = (m + CL - 1) / CL;
-    auto push = [&](int ii, double val) {
-      const int o = ii / ch;
-      cl.map_shared_rank(cp, o)[rank * ch + (ii - o * ch)] = val;
-    };
-    const bool s_in = k > kres, s_out = k >= kres;   // the owned columns are read / written in the slice
-    if (g < G) {
-      const int64_t gst = (int64_t)G * CL * n, sst = (int64_t)G * mres;
-      const int64_t ist = s_in ? sst : gst, ost = s_out ? sst : gst;
-      const int jg = j0 + g * CL;   // the group's first column
-      const int64_t sbase = (int64_t)((jg - myr0) / CL) * mres - kr1;
-      for (int ii = r; ii < m; ii += R) {
-        const int i = k1 + ii;
-        const double vpi = pending ? vp[i] : 0.0, wpi = pending ? wp[i] : 0.0;
-        double acc = 0.0;
-        const double *ia = s_in ? sl + sbase + i : A + (int64_t)jg * n + i;
-        double *oa = s_out ? sl + sbase + i : A + (int64_t)jg * n + i;
-        int q = g;
-        if (pending || s_out != s_in) {
-          // eight loads issued before the eight stores (a store through a
-          // may alias the next load: interleaved, every column would wait
-          // out a full L2 round trip)
-          for (; q + 7 * G < mloc; q += 8 * G, ia += 8 * ist, oa += 8 * ost) {
-            double x[8];
+      __syncthreads();
+      const bool last = L == NB - 1;
+      // eight lanes a row: the row's sums, and those of row k with the totals
+      // (cw: V(k) (W^T v) + W(k) (V^T v), ec: (W^T v).(V^T v))
+      double cw = 0.0, ec = 0.0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = ia[u * ist];
+      for (int u = 0; u < 2; ++u) {
+        const int l = h + 8 * u;
+        if (l < L && q0 + 4 * warp < nq) {
+          cw += rb[l] * cs[l] + rb[NB + l] * cs[NB + l];
+          ec += cs[l] * cs[NB + l];
+        }
+      }
+      // (a warp without rows has nothing to do: its instructions would only be in the others' way)
+      const int qw = q0 + 4 * warp;
+      for (int qb = qw; qb < nq; qb += EIG_THREADS / 8) {
+        const int q = qb + (grp & 3);
+        double P = 0.0, Q = 0.0;
+        double *row = vw + q * TD_LD;
+        if (q < nq) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int j = j0 + (q + u * G) * CL;
-              if (pending) x[u] -= vpi * wp[j] + wpi * vp[j];
-              oa[u * ost] = x[u];
-              acc += x[u] * rv(j);
+          for (int u = 0; u < 2; ++u) {
+            const int l = h + 8 * u;
+            if (l < L) {
+              const double v = row[l], w = row[NB + l];
+              P += v * cs[l] + w * cs[NB + l];
+              Q += v * rb[NB + l] + w * rb[l];
             }
           }
-          for (; q < mloc; q += G, ia += ist, oa += ost) {
-            const int j = j0 + q * CL;
-            double x = *ia;
-            if (pending) x -= vpi * wp[j] + wpi * vp[j];
-            *oa = x;
-            acc += x * rv(j);
+        }
+        if (qb == qw) {
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {
+            P += __shfl_xor_sync(0xffffffffu, P, o);
+            Q += __shfl_xor_sync(0xffffffffu, Q, o);
+            cw += __shfl_xor_sync(0xffffffffu, cw, o);
+            ec += __shfl_xor_sync(0xffffffffu, ec, o);
           }
         } else {
-          for (; q < mloc; q += G, ia += ist) acc += *ia * rv(j0 + q * CL);
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {
+            P += __shfl_xor_sync(0xffffffffu, P, o);
+            Q += __shfl_xor_sync(0xffffffffu, Q, o);
+          }
         }
-        if (G == 1)
-          push(ii, acc);
-        else
-          gp[g * m + ii] = acc;
+        // v_k = 1; v.(A v) from a.(A a), its row k and A's symmetry
+        const double yk = rb[2 * NB] * scl + rb[2 * NB + 1];
+        const double vy = scl * (scl * cs[2 * NB] + rb[2 * NB]) + yk;
+        const double K = 0.5 * t * (t * (vy - 2.0 * ec));
+        const double wk = t * (yk - cw) - K;
+        if (q < nq && h == 0) {
+          const double v = rank + q * CL == k ? 1.0 : me[q] * scl;
+          const double w = t * (ys[q] * scl + rk[q] - P) - K * v;
+          row[L] = v;
+          row[NB + L] = w;
+          me[q] = rk[q] - Q - (v * wk + w);   // not used at the panel's end
+        }
       }
-    }
-    if (G > 1) {
       __syncthreads();
-      for (int ii = tid; ii < m; ii += nt) {
-        double acc = 0.0;
-        for (int c = 0; c < G; ++c) acc += gp[c * m + ii];
-        push(ii, acc);
+      if (last) {
+        // ---- the panel's rank-2 NB update of the owned columns from k on
+        flush(NB);
+        for (int x = tid; x < (nq - q0) * NB; x += EIG_THREADS) {
+          const int q = q0 + x / NB, l = x % NB;
+          Wg[(int64_t)l * n + rank + q * CL] = vw[q * TD_LD + NB + l];
+        }
+        cl.sync();
+        // 8 x 8 tiles (owned columns x rows) by m8n8k4 products over [V | W]: a
+        // warp holds the right-hand factors of 16 rows and takes the owned
+        // columns past them (32 plain multiply-adds an entry would read their
+        // factors from shared memory at 16 bytes a lane: four times as long)
+        const int tr = lane >> 2, tk = lane & 3;
+        for (int ib = k + 16 * warp; ib < n; ib += 16 * NW) {
+          double bv[2][2 * NB / 4];
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const int i = min(ib + 8 * g + tr, n - 1);   // a row past the end is not stored
+            const double *Vp = A + (int64_t)p * n + i, *Wp = Wg + i;
+#pragma unroll
+            for (int u = 0; u < NB / 4; ++u) {
+              bv[g][u] = __ldcg(Vp + (int64_t)(4 * u + tk) * n);
+              bv[g][NB / 4 + u] = __ldcg(Wp + (int64_t)(4 * u + tk) * n);
+            }
+          }
+          for (int q = q0; q < nq; q += 8) {
+            const int qa = min(q + tr, nq - 1);   // nor a column past the last
+            const double *row = vw + qa * TD_LD + tk;
+            double *c0 = qa >= qr ? res(qa) : glo(qa);
+            double c[2][2], av[2 * NB / 4];
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const int i = ib + 8 * g + 2 * tk + u;
+                c[g][u] = i < n ? c0[i] : 0.0;
+              }
+#pragma unroll
+            for (int u = 0; u < NB / 4; ++u) {   // V of the rows meets W of the columns, and W V
+              av[u] = -row[NB + 4 * u];
+              av[NB / 4 + u] = -row[4 * u];
+            }
+#pragma unroll
+            for (int u = 0; u < 2 * NB / 4; ++u)
+#pragma unroll
+              for (int g = 0; g < 2; ++g) td_dmma(c[g], av[u], bv[g][u]);
+            if (q + tr < nq) {
+#pragma unroll
+              for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                  const int i = ib + 8 * g + 2 * tk + u;
+                  if (i < n) c0[i] = c[g][u];
+                }
+            }
+          }
+        }
+        __syncthreads();
+        p = k;
+        fresh = true;
+        if (qr > q0 && (int64_t)(nq - q0) * (n - k) <= cap) {
+          // all owned columns fit from here on
+          for (int q = qr + warp; q < nq; q += NW)
+            for (int i = k + lane; i < n; i += 32) glo(q)[i] = res(q)[i];
+          __syncthreads();
+          qr = q0;
+          st = n - k;
+          r0 = k;
+          for (int q = qr + warp; q < nq; q += NW)
+            for (int i = k + lane; i < n; i += 32) res(q)[i] = glo(q)[i];
+          __syncthreads();
+        }
       }
     }
-    // the cluster barrier's release / acquire order the column writes
-    // (global memory) and the parts (shared memory) for the other CTAs
-    cl.sync();
-    // column k + 1 is complete now (its owner stored it before the barrier):
-    // its loads for the next step overlap the sums below
-    if (k + 2 < n) {
-      const double *c1 = A + (int64_t)k1 * n;
-      if (s_out) {   // in the slice of its owner
-        const int ow = k1 % CL;
-        c1 = cl.map_shared_rank(sl, ow) + (int64_t)((k1 - jr0(ow)) / CL) * mres - kr1;
+    const int jc = k - p;   // the step's column of the panel
+    if (fresh) {
+      for (int q = q0 + tid; q < nq; q += EIG_THREADS) me[q] = q >= qr ? res(q)[k] : glo(q)[k];
+      __syncthreads();
+    }
+    // warp w sends the owned entries to CTA w
+    if (warp < CL && warp != rank) {
+      const uint32_t o = td_remote(td_smem(me), warp), ob = td_remote(bar0, warp);
+      for (int q = q0 + lane; q < nq; q += 32) td_send(o + q * 8, me[q], ob);
+    }
+    if (tid == 0) td_expect(bar0, (uint32_t)(n - k - (nq - q0)) * 8);
+    if (!late) late = !td_wait(bar0, k & 1);
+    if (rank == 0 && tid == 0) de[jc] = col[k % CL * lc + k / CL];
+    if (k == n - 1) break;
+    // ---- the reflector's scale; A a
+    const int k1 = k + 1, q1 = own_from(k1);
+    const int ia = k1 + 1 + lane;   // a starts at row k1 + 1
+    const double *xa = col + ia % CL * lc + ia / CL;
+    if (warp == MW) {
+      const double alpha = col[k1 % CL * lc + k1 / CL];
+      double s4[4] = {0.0, 0.0, 0.0, 0.0};
+      const double *x = xa;
+      int i = ia;
+      for (; i + 96 < n; i += 128, x += 128 / CL) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s4[u] += x[u * (32 / CL)] * x[u * (32 / CL)];
       }
+      for (; i < n; i += 32, x += 32 / CL) s4[0] += *x * *x;
+      double ss = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) {
+        double beta = alpha, t = 0.0, scl = 0.0;
+        if (ss > 0.0) {
+          const double nr = sqrt(alpha * alpha + ss);
+          beta = alpha >= 0.0 ? -nr : nr;
+          t = (beta - alpha) / beta;
+          scl = 1.0 / (alpha - beta);
+        }
+        sc[0] = scl;
+        sc[1] = t;
+        de[NB + jc] = beta;
+        de[2 * NB + jc] = t;
+        stg[2 * NB + MW] = 0.0;
+      }
+    } else {
+      // parts of W^T a and V^T a: column l = warp
+      double dw = 0.0, dv = 0.0, ya = 0.0;
+      bool more = warp < jc;   // dw and dv are still to be summed
+      if (warp < jc)
+        for (int q = own_from(k1 + 1) + lane; q < nq; q += 32) {
+          const double a = me[q];
+          dw += a * vw[q * TD_LD + NB + warp];
+          dv += a * vw[q * TD_LD + warp];
+        }
+      auto batch = [&](auto colptr, int qa, int qe) {
+        for (int qb = qa + warp; qb < qe; qb += 4 * MW) {
+          const double *cp[4];
+          double f[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+          const int nc = min(4, (qe - 1 - qb) / MW + 1);
 #pragma unroll
-      for (int c = 0; c < TD_NX; ++c) {
-        const int i = k1 + tid + c * nt;
-        nx[c] = i < n ? c1[i] : 0.0;
+          for (int c = 0; c < 4; ++c) {
+            cp[c] = colptr(c < nc ? qb + c * MW : qb);
+            f[c] = cp[c][k1];
+          }
+          switch (nc) {
+            case 1: td_dots<1, 32 / CL>(cp, xa, ia, n, acc, more, dw, dv); break;
+            case 2: td_dots<2, 32 / CL>(cp, xa, ia, n, acc, more, dw, dv); break;
+            case 3: td_dots<3, 32 / CL>(cp, xa, ia, n, acc, more, dw, dv); break;
+            default: td_dots<4, 32 / CL>(cp, xa, ia, n, acc, more, dw, dv); break;
+          }
+          more = false;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (c >= nc) break;
+            const int q = qb + c * MW;
+            if (rank + q * CL != k1) ya += acc[c] * me[q];
+            if (lane == 0) {
+              ys[q] = acc[c];
+              rk[q] = f[c];
+            }
+          }
+        }
+      };
+      if (q1 < qr) batch([&](int q) -> const double * { return glo(q); }, q1, qr);
+      batch([&](int q) -> const double * { return res(q); }, max(q1, qr), nq);
+      if (more)
+        for (int o = 16; o > 0; o >>= 1) {
+          dw += __shfl_xor_sync(0xffffffffu, dw, o);
+          dv += __shfl_xor_sync(0xffffffffu, dv, o);
+        }
+      if (lane == 0) {
+        stg[warp] = dw;
+        stg[NB + warp] = dv;
+        stg[2 * NB + warp] = ya;
       }
     }
-    if (owner)
-      for (int i = k1 + tid; i < n; i += nt) colk[i] = rv(i);
-    // CTA c sums the parts of its rows from its bin (in sender order), and
-    // stores the sums into every CTA's pp and its part of p.v into every
-    // CTA's pvs[c]; after the second barrier each CTA reads only its own
-    // shared memory.  Every exchange is a store to another CTA's shared
-    // memory: a store does not wait for its reply as a remote load does.
-    // A bin is written again in the next step's product, after its owner
-    // has passed the second barrier; pp and pvs after the next step's first
-    // barrier, which every reader passes after its reads.
-    const int lo = min(m, rank * ch), hi = min(m, lo + ch);
-    double pv = 0.0;
-    for (int ii = lo + tid; ii < hi; ii += nt) {
-      double p = 0.0;
-#pragma unroll
-      for (int c = 0; c < CL; ++c) p += cp[c * ch + (ii - lo)];
-      p *= t;
-      pv += p * rv(k1 + ii);
-#pragma unroll
-      for (int c = 0; c < CL; ++c) cl.map_shared_rank(pp, c)[ii] = p;
-    }
-    pv = block_sum1(pv, red2, half);
-    if (tid < CL) cl.map_shared_rank(pvs, tid)[rank] = pv;
-    cl.sync();
-    double K = 0.0;
-#pragma unroll
-    for (int c = 0; c < CL; ++c) K += pvs[c];
-    K *= 0.5 * t;
-    for (int ii = tid; ii < m; ii += nt) {
-      const int i = k1 + ii;
-      const double vi = rv(i);
-      wp[i] = pp[ii] - K * vi;
-      vp[i] = vi;
-    }
-    pending = true;
     __syncthreads();
+    // warp w sends the parts, and the owner of row k1 its row, to CTA w
+    if (warp < CL) {
+      const uint32_t o = td_remote(td_smem(part + rank * TD_PL), warp), ob = td_remote(bar1, warp);
+      td_send(o + lane * 8, stg[lane], ob);
+      if (lane < NB) td_send(o + (2 * NB + lane) * 8, stg[2 * NB + lane], ob);
+      if (k1 % CL == rank) {
+        const uint32_t b = td_remote(td_smem(rb), warp);
+        td_send(b + lane * 8, vw[k1 / CL * TD_LD + lane], ob);
+        if (lane < 2) td_send(b + (2 * NB + lane) * 8, (lane ? rk : ys)[k1 / CL], ob);
+      }
+    }
+    if (tid == 0) td_expect(bar1, (CL * TD_PT + TD_LD) * 8);
+    if (!late) late = !td_wait(bar1, k & 1);
   }
-  // the last diagonal entry, from its owner's slice when the last step
-  // wrote it there
-  const bool last_in_slice = n - 2 >= kres;
-  if (last_in_slice && rank == (n - 1) % CL && tid == 0)
-    d[n - 1] = sl[(int64_t)((n - 1 - myr0) / CL) * mres + (n - 1 - kr1)];
+  __syncthreads();
+  flush(n - 1 - p);
+  if (rank == 0 && tid == 0) {
+    d[n - 1] = de[n - 1 - p];
+    tau[n - 1] = 0.0;
+  }
+  if (__syncthreads_or(late)) {
+    // what was not waited for may still be on its way: no CTA leaves at once
+    if (tid == 0) atomicOr(status, 4);
+    const long long c0 = clock64();
+    while (clock64() - c0 < 1000000) {
+    }
+  }
   __threadfence();
-  cl.sync();   // the last parts are read; every owner's writes are visible
-  if (rank == 0) {
-    if (tid == 0) {
-      if (!last_in_slice) d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
-      tau[n - 1] = 0.0;
-    }
-    __syncthreads();
-    tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red2);
-  }
+  cl.sync();   // every owner's writes are visible
+  if (rank == 0) tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red);
 }
 
 // One cluster of CL CTAs per entry of the cluster list: a large sector
@@ -477,19 +711,20 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
     tridiag_kernel(double *Aall, const int64_t *off, const int *dims, const int64_t *eoff, const int *tsec,
-                   const int *tbig, double *dall, double *eall, double *tauall, double *info, double *dsall, double *e2all,
-                   int64_t smem_doubles) {
-  extern __shared__ double sm[];
-  __shared__ double red[64];
-  __shared__ double sh_tau, sh_scl, sh_pvs[16];
+                   const int *tbig, double *dall, double *eall, double *tauall, double *Wall, double *info,
+                   double *dsall, double *e2all, int64_t smem_doubles, int *status) {
+  extern __shared__ __align__(16) double td_sm[];
+  __shared__ double red[48];
+  __shared__ double sh_tau, sh_scl;
+  __shared__ uint64_t mbar[2];
   cg::cluster_group cl = cg::this_cluster();
   const int b = blockIdx.x / CL, rank = (int)cl.block_rank();
   const int s = tsec[blockIdx.x];
   if (tbig[b]) {
-    tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, sm, smem_doubles, red,
-                     sh_pvs);
+    tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, Wall, info, dsall, e2all, td_sm, smem_doubles,
+                     red, mbar, status);
   } else if (s >= 0 && dims[s] > 0) {
-    tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, sm, red, sh_tau, sh_scl);
+    tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, td_sm, red, sh_tau, sh_scl);
   }
 }
 
@@ -1484,7 +1719,8 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return dims[a] > dims[b]; });
     // trD: d, e, tau, eigenvalues, scaled d, scaled e^2 (etot each), then 4 per sector
-    if ((rc = ctx->trB.reserve(sizeof(double) * (rlen + 4))) ||
+    // trB: rho by sector, then the panel matrix W of each (TD_NB rows)
+    if ((rc = ctx->trB.reserve(sizeof(double) * (rlen + TD_NB * etot + 4))) ||
         (rc = ctx->trD.reserve(sizeof(double) * (6 * etot + 4 * nsec + 8))))
       return rc;
     double *dd = ctx->trD.d(), *de = dd + etot, *dtau = de + etot, *dev = dtau + etot, *dds = dev + etot,
@@ -1493,8 +1729,10 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     // small sectors tcl at a time (largest first)
     // shared memory: the per-sector vectors, and for a sector reduced by a
     // cluster as much more as a CTA may have (its slice of the trailing block)
-    size_t tsm = sizeof(double) * (6 * (size_t)maxn + std::max(maxn, EIG_THREADS));
+    const int maxs = std::min(maxn, TD_BIG - 1);
+    size_t tsm = sizeof(double) * (3 * (size_t)maxs + std::max(maxs, EIG_THREADS));
     if (maxn >= TD_BIG) {
+      tsm = std::max(tsm, sizeof(double) * (size_t)td_coop_doubles(maxn, 8));
       int optin = 0;
       cudaFuncAttributes fa;
       if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
@@ -1525,13 +1763,14 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     const size_t p_roff = tab.add(roff), p_eoff = tab.add(eoff), p_dims = tab.add(dims), p_tsec = tab.add(tsec);
     const size_t p_tbig = tab.add(tbig), p_esec = tab.add(esec), p_cnt = tab.zeros(256);
     const int ndot = dot_blocks(D);
-    const size_t p_part = tab.room(sizeof(double) * (ndot + 1));   // partial sums of |psi|^2, then |psi|^2
+    const size_t p_part = tab.room(sizeof(double) * ndot);   // partial sums of |psi|^2
     if ((rc = ctx->trE.reserve(tab.size())) || (rc = ctx->trC.reserve(sizeof(double) * (nslots * BM * BN + 4)))) return rc;
     char *tbase = (char *)ctx->trE.p;
     CKT(cudaMemcpyAsync(tbase, tab.buf.data(), tab.buf.size(), cudaMemcpyHostToDevice, st));
     const int64_t *d_roff = (const int64_t *)(tbase + p_roff), *d_eoff = (const int64_t *)(tbase + p_eoff);
     const int *d_dims = (const int *)(tbase + p_dims);
     int *d_status = (int *)(tbase + p_cnt + 16);
+    double *d_nrm2 = (double *)(tbase + p_cnt + 8);   // |psi|^2, before the status words
     GemmParams g;
     std::memset(&g, 0, sizeof g);
     g.psi = psi;
@@ -1545,7 +1784,7 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     g.slots = ctx->trC.d();
     double *part = (double *)(tbase + p_part);
     launch_dot(psi, psi, D, part, ndot, st);
-    rho_scale_kernel<<<1, 256, 0, st>>>(part, ndot, (Task *)(tbase + p_tasks), (int)tasks.size(), part + ndot);
+    rho_scale_kernel<<<1, 256, 0, st>>>(part, ndot, (Task *)(tbase + p_tasks), (int)tasks.size(), d_nrm2);
     launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
     launch_reduce(g, (const Reduce *)(tbase + p_red), (int)red.size(), st);
     CKT(cudaGetLastError());
@@ -1556,11 +1795,13 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       if (tcl == 16) {
         CKT(cudaFuncSetAttribute(tridiag_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<16><<<nclus * 16, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
-                                                                 dd, de, dtau, dinfo, dds, de2, (int64_t)(tsm / 8));
+                                                                 dd, de, dtau, ctx->trB.d() + rlen, dinfo, dds, de2, (int64_t)(tsm / 8),
+        d_status);
       } else {
         CKT(cudaFuncSetAttribute(tridiag_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<8><<<nclus * 8, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
-                                                               dd, de, dtau, dinfo, dds, de2, (int64_t)(tsm / 8));
+                                                               dd, de, dtau, ctx->trB.d() + rlen, dinfo, dds, de2, (int64_t)(tsm / 8),
+        d_status);
       }
       CKT(cudaGetLastError());
     }
@@ -1571,11 +1812,13 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       CKT(cudaGetLastError());
     }
     std::vector<double> ev(etot);
-    CKT(cudaMemcpyAsync(ctx->pinned, part + ndot, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CKT(cudaMemcpyAsync(ctx->pinned, d_nrm2, 16, cudaMemcpyDeviceToHost, st));   // and the status word
     CKT(cudaMemcpyAsync(ev.data(), dev, sizeof(double) * etot, cudaMemcpyDeviceToHost, st));
     CKT(cudaEventRecord(ctx->tev[3], st));
     CKT(cudaStreamSynchronize(st));
     const double nrm2 = ctx->pinned[0];
+    if (reinterpret_cast<const int *>(ctx->pinned + 1)[0] & 4)
+      return set_err(TJ_ERR_TIMEOUT, "tj_truncation: a wait of the tridiagonal reduction gave up");
     if (!(nrm2 > 0) || !std::isfinite(nrm2)) return set_err(TJ_ERR_NUMERIC, "tj_truncation: zero or non-finite psi");
     const auto sel0 = std::chrono::steady_clock::now();
     float stage_ms[7] = {0, 0, 0, 0, 0, 0, 0};
