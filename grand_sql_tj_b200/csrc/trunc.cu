@@ -46,11 +46,13 @@ constexpr int EIG_MAX_N = 4096;
 constexpr double EIG_EPS = 2.220446049250313e-16;        // 2^-52
 constexpr double EIG_SAFMIN = 2.2250738585072014e-308;   // smallest normal FP64
 constexpr int ORTH_THREADS = 512;
-// Sectors of at least this many states are reduced by a whole cluster: alone,
-// 191 states take 0.84 ms in one CTA, 192 take 0.56 in a cluster, 261 1.77 and 0.78,
-// 319 2.98 and 1.00; but only seven clusters of 16 run at a time, so the line
-// lies above the break-even of one sector.
-constexpr int TD_BIG = 192;
+// A sector of up to TD_SMALL states is reduced in one CTA's shared memory (62
+// states: 87 us, 133 from L2; with three rows a lane 96 would take 248 and 238,
+// with five 160 720 and 558), one of at least TD_BIG by a whole cluster: alone, 191 states
+// take 0.84 ms in one CTA, 192 take 0.54 in a cluster, 261 1.77 and 0.75, 319 2.98
+// and 0.95; but only seven clusters of 16 run at a time, so the line lies above
+// the break-even of one sector (14 sectors of 180: 0.74 ms and 1.01).
+constexpr int TD_SMALL = 64, TD_BIG = 192;
 
 // Sum of the warps' partial sums r[0..nw-1] by every warp: lane w takes
 // r[w] and a shuffle tree adds them, in the same order in every warp (a
@@ -78,11 +80,8 @@ __device__ __forceinline__ double block_sum(double x, double *red) {
 // k+1..n-1 and v_k(k+1) = 1 (the lower-triangle scheme of LAPACK's dsytd2).
 // v_k overwrites A(k+1:n, k); d and e receive the diagonal and the
 // off-diagonal of T, info[4s..4s+3] its Gershgorin interval, max row sum and
-// the Sturm-count pivot floor.  The rank-2 update of step k,
-// A <- A - v w^T - w v^T, is applied lazily inside the matrix-vector product
-// p = A v of step k+1, so each step reads and writes the trailing block once.
-// One CTA per sector (tridiag_one) or one cluster per large sector
-// (tridiag_coop).
+// the Sturm-count pivot floor.  One CTA per sector (tridiag_small, tridiag_one)
+// or one cluster per large sector (tridiag_coop).
 // By all threads of one CTA: info, and the scaled diagonal ds and squared
 // off-diagonal e2 that the Sturm counts read.  red: 48 doubles.
 __device__ void tridiag_info(int s, int n, const double *d, const double *e, double *info, double *ds, double *e2,
@@ -127,6 +126,144 @@ __device__ void tridiag_info(int s, int n, const double *d, const double *e, dou
 }
 static_assert(EIG_THREADS <= 512, "tridiag_info's scratch");
 
+// One sector of up to 32 C states by one CTA, the matrix in shared memory.  Each
+// warp keeps the whole reflector and the pending w, row lane + 32 c in register
+// c of a lane, and owns the columns j = warp (mod NW): the rank-2 update of step
+// k - 1, A <- A - v w^T - w v^T, is applied to them as they are read for
+// p = A v of step k, whose entry j is (A being symmetric) the product of column
+// j with v.  Every warp finds the reflector of column k and, from p, the new w
+// for itself, so a step has one CTA barrier; the parts are a chain of three sums
+// over a warp, a square root and a division, and the warps' instructions, most
+// of them the same in each: NW = 8 of the CTA's 16 take part (62 states: 125 us
+// with 4, 87 with 8, 96 with 16; the load of a column behind the store of the
+// one before: 97).
+template <int C, int NW>
+__device__ void tridiag_small(int s, double *Aall, const int64_t *off, const int *dims, const int64_t *eoff,
+                              double *dall, double *eall, double *tauall, double *info, double *dsall,
+                              double *e2all, double *sm, double *red) {
+  const int n = dims[s], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *A = Aall + off[s];
+  double *d = dall + eoff[s], *e = eall + eoff[s], *tau = tauall + eoff[s];
+  double *L = sm, *p = sm + n * n;   // p: two of n, by the parity of the step
+  for (int x = tid; x < n * n; x += EIG_THREADS) L[x] = A[x];
+  double vp[C], wp[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) vp[c] = wp[c] = 0.0;
+  // entry j of a vector held as above
+  auto at = [&](const double (&x)[C], int j) {
+    double y = x[0];
+#pragma unroll
+    for (int c = 1; c < C; ++c) y = (j >> 5) == c ? x[c] : y;
+    return __shfl_sync(0xffffffffu, y, j & 31);
+  };
+  auto wsum = [](double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  __syncthreads();
+  for (int k = 0; k + 1 < n && warp < NW; ++k) {
+    const int k1 = k + 1;
+    const double wk = at(wp, k), vk = at(vp, k);
+    double v[C], ss = 0.0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int i = lane + 32 * c;
+      v[c] = i >= k && i < n ? L[k * n + i] - (vp[c] * wk + wp[c] * vk) : 0.0;
+      if (i > k1) ss += v[c] * v[c];
+    }
+    ss = wsum(ss);
+    const double dk = at(v, k), alpha = at(v, k1);
+    double beta = alpha, t = 0.0, scl = 0.0;
+    if (ss > 0.0) {
+      const double nr = sqrt(alpha * alpha + ss);
+      beta = alpha >= 0.0 ? -nr : nr;
+      t = (beta - alpha) / beta;
+      scl = 1.0 / (alpha - beta);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int i = lane + 32 * c;
+      v[c] = i > k1 ? v[c] * scl : i == k1 ? 1.0 : 0.0;
+    }
+    if (warp == k % NW) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int i = lane + 32 * c;
+        if (i >= k1 && i < n) A[k * n + i] = v[c];
+      }
+      if (lane == 0) {
+        d[k] = dk;
+        e[k] = beta;
+        tau[k] = t;
+      }
+    }
+    double *pk = p + (k & 1) * n;
+    for (int j0 = k1 + ((warp - k1) % NW + NW) % NW; j0 < n; j0 += 4 * NW) {
+      // four columns' loads before their stores, which may alias them
+      double acc[4], x[4][C];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double *Lj = L + (j0 + u * NW) * n + lane;
+        const int top = j0 + u * NW < n ? n : 0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) x[u][c] = lane + 32 * c >= k1 && lane + 32 * c < top ? Lj[32 * c] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = min(j0 + u * NW, n - 1);
+        const double wj = at(wp, j), vj = at(vp, j);
+        acc[u] = 0.0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          x[u][c] -= vp[c] * wj + wp[c] * vj;
+          acc[u] += x[u][c] * v[c];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        double *Lj = L + (j0 + u * NW) * n + lane;
+        const int top = j0 + u * NW < n ? n : 0;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          if (lane + 32 * c >= k1 && lane + 32 * c < top) Lj[32 * c] = x[u][c];
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (lane == 0 && j0 + u * NW < n) pk[j0 + u * NW] = acc[u];
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
+    double pv = 0.0, q[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int i = lane + 32 * c;
+      q[c] = i >= k1 && i < n ? t * pk[i] : 0.0;
+      pv += q[c] * v[c];
+    }
+    const double K = 0.5 * t * wsum(pv);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      wp[c] = q[c] - K * v[c];
+      vp[c] = v[c];
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    d[n - 1] = L[n * n - 1];   // the last reflector is none: nothing is pending
+    tau[n - 1] = 0.0;
+  }
+  __syncthreads();
+  tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red);
+}
+
+// One sector too large for tridiag_small by one CTA, the matrix in L2: the
+// rank-2 update of step k, A <- A - v w^T - w v^T, is applied inside the
+// product p = A v of step k + 1, so each step reads and writes the trailing
+// block once.
 __device__ void tridiag_one(int s, double *Aall, const int64_t *off, const int *dims, const int64_t *eoff,
                             double *dall, double *eall, double *tauall, double *info, double *dsall, double *e2all,
                             double *sm, double *red, double &sh_tau, double &sh_scl) {
@@ -724,7 +861,13 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
     tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, Wall, info, dsall, e2all, td_sm, smem_doubles,
                      red, mbar, status);
   } else if (s >= 0 && dims[s] > 0) {
-    tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, td_sm, red, sh_tau, sh_scl);
+    const int n = dims[s];
+    if (n <= 32)
+      tridiag_small<1, 8>(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, td_sm, red);
+    else if (n <= TD_SMALL)
+      tridiag_small<TD_SMALL / 32, 8>(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, td_sm, red);
+    else
+      tridiag_one(s, Aall, off, dims, eoff, dall, eall, tauall, info, dsall, e2all, td_sm, red, sh_tau, sh_scl);
   }
 }
 
@@ -1727,10 +1870,12 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
            *de2 = dds + etot, *dinfo = de2 + etot;
     // clusters of the tridiagonal reduction: one per large sector, then the
     // small sectors tcl at a time (largest first)
-    // shared memory: the per-sector vectors, and for a sector reduced by a
-    // cluster as much more as a CTA may have (its slice of the trailing block)
-    const int maxs = std::min(maxn, TD_BIG - 1);
-    size_t tsm = sizeof(double) * (3 * (size_t)maxs + std::max(maxs, EIG_THREADS));
+    // shared memory: a small sector's matrix, a middle one's vectors; for one
+    // reduced by a cluster as much as a CTA may have (its columns)
+    size_t tsm = 0;
+    for (int n : dims)
+      if (n < TD_BIG)
+        tsm = std::max(tsm, sizeof(double) * (n <= TD_SMALL ? (size_t)n * (n + 2) : 3 * (size_t)n + EIG_THREADS));
     if (maxn >= TD_BIG) {
       tsm = std::max(tsm, sizeof(double) * (size_t)td_coop_doubles(maxn, 8));
       int optin = 0;

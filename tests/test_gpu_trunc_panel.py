@@ -1,5 +1,6 @@
-"""The panelled tridiagonal reduction of a large sector: whole and partial last
-panels, owned columns that are all, partly or from some panel on resident, and
+"""The tridiagonal reductions: of a small sector in one CTA's shared memory at
+the row counts of its lanes; the panelled one of a large sector: whole and
+partial last panels, owned columns that are all, partly or from some panel on resident, and
 the smallest trailing blocks a cluster shares; the tolerances are those of the
 truncation's other stages (a backward error of 20 n eps ||rho||).
 """
@@ -17,11 +18,18 @@ def test_panels(ctx, n, kept):  # noqa: F811
     _check(ctx, _psi(n, n, np.exp(-4.0 * np.arange(n) / n), n), kept)
 
 
-@pytest.mark.parametrize("n", [330, 660])
+# by one CTA: in shared memory, one or two rows a lane; above 64 states in L2
+@pytest.mark.parametrize("n,kept", [(1, 1), (2, 2), (3, 3), (16, 9), (17, 17), (32, 32), (33, 20), (64, 64), (65, 30), (96, 96),
+                                    (97, 50), (128, 128), (159, 70), (160, 160)])
+def test_one_cta(ctx, n, kept):  # noqa: F811
+    _check(ctx, _psi(n, n, np.exp(-4.0 * np.arange(n) / n), n), kept)
+
+
+@pytest.mark.parametrize("n", [150, 330, 660])
 def test_panels_deflate(ctx, n):  # noqa: F811
     """Reflectors that vanish: a matrix that is diagonal but for a block."""
     rng = np.random.default_rng(n)
     d = np.diag(rng.uniform(0.1, 1.0, n))
-    d[100:140, 100:140] = rng.standard_normal((40, 40))
+    d[60:100, 60:100] = rng.standard_normal((40, 40))
     d[n - 30:, n - 30:] = 0.0
     _check(ctx, d, n // 3)
