@@ -949,11 +949,13 @@ extern "C" int tj_get_hamiltonian(tj_ctx *ctx, const tj_lattice *lat, int side, 
   if ((rc = ctx->side_stream(0, up)) || (rc = ctx->side_stream(1, down)) || (rc = ctx->reserve_events(3 * K + 1)))
     return rc;
   struct Join {
-    cudaStream_t a, b, c;
-    ~Join() {   // nothing is left running, on any way out
-      cudaStreamSynchronize(a);
-      cudaStreamSynchronize(b);
-      cudaStreamSynchronize(c);
+    cudaStream_t up, st, down;
+    bool done = false;
+    ~Join() {   // nothing of the steps is left running, on any way out
+      if (done) return;
+      cudaStreamSynchronize(up);
+      cudaStreamSynchronize(st);
+      cudaStreamSynchronize(down);
     }
   } join{up, st, down};
   cudaPointerAttributes pa;
@@ -1044,7 +1046,8 @@ extern "C" int tj_get_hamiltonian(tj_ctx *ctx, const tj_lattice *lat, int side, 
     return rc;
   }
   CKR(cudaEventRecord(ctx->ev[2], st));
-  CKR(cudaStreamSynchronize(st));
+  CKR(cudaStreamSynchronize(st));   // behind the last step, which waited for the copies in, and the copies out
+  join.done = true;
   float gemm_ms = 0, all_ms = 0;
   for (int c = 0; c < K; ++c) {   // the steps' products (their waits for copies are between them)
     float ms = 0;
