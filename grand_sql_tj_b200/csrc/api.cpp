@@ -56,23 +56,13 @@ tj_ctx::~tj_ctx() {
   for (auto &e : tev)
     if (e) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
-  for (auto &e : events) cudaEventDestroy(e);
-  for (auto &s : side)
-    if (s) cudaStreamDestroy(s);
+  if (side) cudaStreamDestroy(side);
   if (pinned) cudaFreeHost(pinned);
 }
 
-int tj_ctx::side_stream(int i, cudaStream_t &s) {
-  if (!side[i]) CK(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
-  s = side[i];
-  return TJ_OK;
-}
-int tj_ctx::reserve_events(size_t n) {
-  while (events.size() < n) {
-    cudaEvent_t e;
-    CK(cudaEventCreate(&e));
-    events.push_back(e);
-  }
+int tj_ctx::side_stream(cudaStream_t &s) {
+  if (!side) CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  s = side;
   return TJ_OK;
 }
 
@@ -698,7 +688,7 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   auto ref = [&](int off) { return LzRef{V, ld, itd, off, nullptr}; };
   const bool is_short = lz_short(D);
   cudaStream_t side = nullptr;
-  if (is_short && (rc = ctx->side_stream(0, side))) return rc;
+  if (is_short && (rc = ctx->side_stream(side))) return rc;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));

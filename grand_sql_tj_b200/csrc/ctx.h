@@ -68,10 +68,8 @@ struct tj_ctx {
   cudaStream_t stream = nullptr;
   // work beside the main stream's, made at its first use; whoever uses it
   // orders it by events and leaves nothing running on it at return
-  cudaStream_t side[2] = {nullptr, nullptr};
-  int side_stream(int i, cudaStream_t &s);
-  std::vector<cudaEvent_t> events;   // for such orderings, with timing
-  int reserve_events(size_t n);
+  cudaStream_t side = nullptr;
+  int side_stream(cudaStream_t &s);
   double *pinned = nullptr;   // 32 doubles of page-locked host memory for scalar read-backs
   // H*psi timing: 0 start, 1 after the splits of psi, 2 after the first GEMM
   // launch, 3 after the product splits, 4 end (FP64: 1 = 0 and 3 = 2)

@@ -521,138 +521,7 @@ struct RenormPlan {
   int len = 0, nsub = 0;
   int64_t out_len = 0;
   uint64_t key = 0;
-  // The pass over the operators in steps: the ends of each step's uploads,
-  // tiles and reduce records, and the part of the result complete after it.
-  struct Step {
-    int up = 0, tile1 = 0, red1 = 0, tile2 = 0, red2 = 0;
-    std::vector<std::pair<int64_t, int64_t>> out;   // (offset, doubles)
-  };
-  std::vector<Step> steps;
 };
-
-// Cuts the pass into steps along the uploads, so that the copies in, the
-// products and the copies out of different steps run at the same time: a
-// product goes to the step that uploads the last of its operands, and the
-// result is cut into parts that are copied out after the step that completes
-// them.  A step carries at least RN_STEP bytes in (at 54 GB/s 80 us, against
-// some 20 us of launches and last waves of a step's products), and there are at
-// most RN_STEPS.
-constexpr int64_t RN_STEP = (int64_t)4 << 20, RN_STEPS = 8;
-static void cut_steps(RenormPlan &R) {
-  HpsiPlan &P = R.P;
-  int64_t total = 0;
-  for (const auto &u : P.uploads) total += u.n;
-  const int K = (int)std::max<int64_t>(1, std::min<int64_t>(RN_STEPS, 8 * total / RN_STEP));
-  R.steps.assign(K, RenormPlan::Step());
-  if (K == 1) {
-    R.steps[0] = {(int)P.uploads.size(), (int)P.tiles1.size(), (int)P.red1.size(), (int)P.tiles2.size(),
-                  (int)P.red2.size(), {{0, R.out_len}}};
-    return;
-  }
-  auto op_upload = [&](int64_t off) {   // the upload that holds a place of the operator storage
-    return (int)(std::upper_bound(P.uploads.begin(), P.uploads.end(), off,
-                                  [](int64_t x, const HpsiPlan::Upload &u) { return x < u.dst; }) -
-                 P.uploads.begin()) - 1;
-  };
-  // the upload that each product (or each task of the result) waits for, -1 for
-  // none; products in the order of their places in scratch; first[b]: the first
-  // one at or past place b << 12
-  std::vector<int> c1(P.cells1.size(), -1), c2(P.cells2.size(), -1);
-  std::vector<int> first((P.scratch_len >> 12) + 2, (int)P.cells1.size());
-  for (size_t i = P.cells1.size(); i-- > 0;) {
-    if (i && P.cells1[i].off < P.cells1[i - 1].off) throw RenormError(TJ_ERR_ARG, "products out of order");
-    first[(P.cells1[i].off + 4095) >> 12] = (int)i;
-  }
-  for (size_t b = first.size() - 1; b-- > 0;) first[b] = std::min(first[b], first[b + 1]);
-  auto need = [&](const Operand &o) {
-    if (o.space == SP_OPS) return op_upload(o.off);
-    if (o.space != SP_SCR) return -1;
-    const size_t b = (size_t)(o.off >> 12);
-    const auto it = std::upper_bound(P.cells1.begin() + first[b], P.cells1.begin() + first[b + 1], o.off,
-                                     [](int64_t x, const Cell &c) { return x < c.off; });
-    return c1[it - P.cells1.begin() - 1];   // the last product at or before the place
-  };
-  for (size_t i = 0; i < P.cells1.size(); ++i) {   // one operator each
-    const Task &t = P.tasks1[P.cells1[i].t_begin];
-    c1[i] = std::max(need(t.L), need(t.R));
-  }
-  std::vector<int> t2(P.tasks2.size());
-  for (size_t t = 0; t < t2.size(); ++t) t2[t] = std::max(need(P.tasks2[t].L), need(P.tasks2[t].R));
-  // uploads in the order in which the result's operators want them, the
-  // Hamiltonian (its first block, which wants most) last; a block that nothing
-  // wants any more (its site has lost its last bond) is not uploaded
-  const int64_t ham_end = R.blocks[0].num < (int)R.recs.size() ? R.recs[R.blocks[0].num].off : R.out_len;
-  size_t nham = 0;
-  while (nham < P.cells2.size() && P.cells2[nham].off < ham_end) ++nham;
-  std::vector<HpsiPlan::Upload> ups;
-  std::vector<int> rank(P.uploads.size(), -1);
-  auto want = [&](int u) {
-    if (u < 0 || rank[u] >= 0) return;
-    rank[u] = (int)ups.size();
-    ups.push_back(P.uploads[u]);
-  };
-  for (size_t i = nham; i < P.cells2.size(); ++i)
-    for (int t = P.cells2[i].t_begin; t < P.cells2[i].t_end; ++t) want(t2[t]);
-  for (size_t i = 0; i < nham; ++i)
-    for (int t = P.cells2[i].t_begin; t < P.cells2[i].t_end; ++t) want(t2[t]);
-  int64_t used = 0;
-  for (const auto &u : ups) used += u.n;
-  std::vector<int> step_of(ups.size());   // by place in the new order
-  {
-    int64_t acc = 0;
-    size_t u = 0;
-    for (int c = 0; c < K; ++c) {
-      for (; u < ups.size() && (c == K - 1 || acc < used * (c + 1) / K); ++u) {
-        acc += ups[u].n;
-        step_of[u] = c;
-      }
-      R.steps[c].up = (int)u;
-    }
-  }
-  auto to_step = [&](int &u) { u = u < 0 ? 0 : step_of[rank[u]]; };
-  // a product that nothing reads waits for the last step (there is none now)
-  for (int &u : c1) {
-    if (u >= 0 && rank[u] < 0) u = K - 1;
-    else to_step(u);
-  }
-  for (int &u : t2) to_step(u);
-  P.uploads.swap(ups);
-  // the result's parts: cells in result order, at least a 32nd of it each;
-  // neighbours that are complete after the same step are one
-  int64_t from = 0;
-  int last = -1;   // the step of the part before
-  for (size_t i = 0, b = 0; i < P.cells2.size(); ++i) {
-    const Cell &c = P.cells2[i];
-    for (int t = c.t_begin; t < c.t_end; ++t) c2[i] = std::max(c2[i], t2[t]);
-    const bool end2 = i + 1 == P.cells2.size();
-    const int64_t to = end2 ? R.out_len : P.cells2[i + 1].off;
-    if (!end2 && to - from < R.out_len / 32) continue;
-    const int step = *std::max_element(c2.begin() + b, c2.begin() + i + 1);
-    std::fill(c2.begin() + b, c2.begin() + i + 1, step);
-    if (step == last)
-      R.steps[step].out.back().second += to - from;
-    else
-      R.steps[step].out.push_back({from, to - from});
-    last = step;
-    from = to;
-    b = i + 1;
-  }
-  if (from < R.out_len) R.steps[K - 1].out.push_back({from, R.out_len - from});   // no cells: zeros
-  // tiles and reduce records by step, their order within one kept (heaviest first)
-  auto group = [&](auto &v, const std::vector<int> &cs, auto mark) {
-    std::vector<int> at(K + 1, 0);
-    for (const auto &x : v) ++at[cs[x.cell] + 1];
-    for (int c = 0; c < K; ++c) at[c + 1] += at[c];
-    for (int c = 0; c < K; ++c) mark(R.steps[c], at[c + 1]);
-    auto w = v;
-    for (const auto &x : v) w[at[cs[x.cell]]++] = x;
-    v.swap(w);
-  };
-  group(P.tiles1, c1, [](RenormPlan::Step &s, int n) { s.tile1 = n; });
-  group(P.red1, c1, [](RenormPlan::Step &s, int n) { s.red1 = n; });
-  group(P.tiles2, c2, [](RenormPlan::Step &s, int n) { s.tile2 = n; });
-  group(P.red2, c2, [](RenormPlan::Step &s, int n) { s.red2 = n; });
-}
 
 int build_renorm_plan(const tj_lattice *lat, int side, int mshift, const tj_model *pre, const tj_basis *basis,
                       const tj_block *trunb, RenormPlan &R, std::string &msg) {
@@ -827,7 +696,6 @@ int build_renorm_plan(const tj_lattice *lat, int side, int mshift, const tj_mode
     P.bytes = bytes + 8.0 * (P.psi_len + R.out_len);
     split_tiles(P.cells1, P.tasks1, P.tiles1, P.red1, P.nslots1, false);
     split_tiles(P.cells2, P.tasks2, P.tiles2, P.red2, P.nslots2, false);
-    cut_steps(R);
     return TJ_OK;
   } catch (const RenormError &e) {
     msg = e.what();
@@ -942,43 +810,14 @@ extern "C" int tj_get_hamiltonian(tj_ctx *ctx, const tj_lattice *lat, int side, 
       (rc = ctx->rnSlots.reserve(sizeof(double) * (std::max(P.nslots1, P.nslots2) * BM * BN + 4))))
     return rc;
   const double pre_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
-  // the copies in on one stream, the products on the context's, the copies out
-  // on another (into page-locked memory; else staged at the end)
-  cudaStream_t up, down;
-  const int K = (int)R.steps.size();
-  if ((rc = ctx->side_stream(0, up)) || (rc = ctx->side_stream(1, down)) || (rc = ctx->reserve_events(3 * K + 1)))
-    return rc;
-  struct Join {
-    cudaStream_t up, st, down;
-    bool done = false;
-    ~Join() {   // nothing of the steps is left running, on any way out
-      if (done) return;
-      cudaStreamSynchronize(up);
-      cudaStreamSynchronize(st);
-      cudaStreamSynchronize(down);
-    }
-  } join{up, st, down};
-  cudaPointerAttributes pa;
-  const bool locked = cudaPointerGetAttributes(&pa, out->data) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-  cudaGetLastError();
   CKR(cudaEventRecord(ctx->ev[5], st));
-  CKR(cudaStreamWaitEvent(up, ctx->ev[5], 0));
+  for (const auto &u : P.uploads)
+    if (u.n > 0) CKR(upload(ctx, ctx->rnOps.d() + u.dst, u.src, u.n, st));
   {
     int64_t lo = LLONG_MAX;
     for (int k = 0; k < trun->num; ++k) lo = std::min(lo, (int64_t)trun->sub[k].off);
-    CKR(upload(ctx, ctx->rnTrun.d(), trun->data + lo, P.psi_len, up));
+    CKR(upload(ctx, ctx->rnTrun.d(), trun->data + lo, P.psi_len, st));
   }
-  auto copy_in = [&](int c) -> int {   // step c's operators
-    for (int i = c ? R.steps[c - 1].up : 0; i < R.steps[c].up; ++i) {
-      const auto &u = P.uploads[i];
-      if (u.n > 0) CKR(upload(ctx, ctx->rnOps.d() + u.dst, u.src, u.n, up));
-    }
-    CKR(cudaEventRecord(ctx->events[3 * c], up));
-    return TJ_OK;
-  };
-  // the first step's before the tables are put together, the others after the
-  // tables' own copy, which would wait for them
-  if ((rc = copy_in(0))) return rc;
   std::vector<char> tab;
   auto add = [&](const void *p, size_t n) {
     size_t at = (tab.size() + 255) / 256 * 256;
@@ -1005,55 +844,31 @@ extern "C" int tj_get_hamiltonian(tj_ctx *ctx, const tj_lattice *lat, int side, 
   g.ops = ctx->rnOps.d();
   g.psi = ctx->rnTrun.d();
   g.scr = ctx->rnScr.d();
+  g.out = ctx->rnScr.d();
+  g.cells = (const Cell *)(tb + o_c1);
+  g.tasks = (const Task *)(tb + o_t1);
+  g.tiles = (const Tile *)(tb + o_l1);
+  g.ntiles = (int)P.tiles1.size();
+  g.counter = (unsigned int *)(tb + o_cnt);
   g.slots = ctx->rnSlots.d();
-  RenormPlan::Step s0;   // the ends of the step before
-  for (int c = 0; c < K; ++c) {
-    const RenormPlan::Step &s = R.steps[c];
-    if (c && (rc = copy_in(c))) return rc;
-    cudaEvent_t *e = &ctx->events[3 * c];
-    CKR(cudaStreamWaitEvent(st, e[0], 0));
-    CKR(cudaEventRecord(e[1], st));
-    g.out = ctx->rnScr.d();
-    g.cells = (const Cell *)(tb + o_c1);
-    g.tasks = (const Task *)(tb + o_t1);
-    g.tiles = (const Tile *)(tb + o_l1) + s0.tile1;
-    g.ntiles = s.tile1 - s0.tile1;
-    g.counter = (unsigned int *)(tb + o_cnt);
-    if (g.ntiles) launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
-    launch_reduce(g, (const Reduce *)(tb + o_r1) + s0.red1, s.red1 - s0.red1, st);
-    g.out = ctx->rnOut.d();
-    g.cells = (const Cell *)(tb + o_c2);
-    g.tasks = (const Task *)(tb + o_t2);
-    g.tiles = (const Tile *)(tb + o_l2) + s0.tile2;
-    g.ntiles = s.tile2 - s0.tile2;
-    g.counter = (unsigned int *)(tb + o_cnt) + 1;
-    if (g.ntiles) launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
-    launch_reduce(g, (const Reduce *)(tb + o_r2) + s0.red2, s.red2 - s0.red2, st);
-    CKR(cudaEventRecord(e[2], st));
-    CKR(cudaGetLastError());
-    if (locked) {
-      CKR(cudaStreamWaitEvent(down, e[2], 0));
-      for (const auto &o : s.out)
-        CKR(cudaMemcpyAsync(out->data + o.first, ctx->rnOut.d() + o.first, sizeof(double) * o.second,
-                            cudaMemcpyDeviceToHost, down));
-    }
-    s0 = s;
-  }
-  if (locked) {
-    CKR(cudaEventRecord(ctx->events[3 * K], down));
-    CKR(cudaStreamWaitEvent(st, ctx->events[3 * K], 0));
-  } else if ((rc = download(ctx, out->data, ctx->rnOut.d(), R.out_len, st))) {
-    return rc;
-  }
+  CKR(cudaEventRecord(ctx->ev[0], st));
+  launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
+  launch_reduce(g, (const Reduce *)(tb + o_r1), (int)P.red1.size(), st);
+  g.out = ctx->rnOut.d();
+  g.cells = (const Cell *)(tb + o_c2);
+  g.tasks = (const Task *)(tb + o_t2);
+  g.tiles = (const Tile *)(tb + o_l2);
+  g.ntiles = (int)P.tiles2.size();
+  g.counter = (unsigned int *)(tb + o_cnt) + 1;
+  launch_grouped_gemm(g, grouped_gemm_grid(g.ntiles), st);
+  launch_reduce(g, (const Reduce *)(tb + o_r2), (int)P.red2.size(), st);
+  CKR(cudaEventRecord(ctx->ev[1], st));
+  CKR(cudaGetLastError());
+  if ((rc = download(ctx, out->data, ctx->rnOut.d(), R.out_len, st))) return rc;
   CKR(cudaEventRecord(ctx->ev[2], st));
-  CKR(cudaStreamSynchronize(st));   // behind the last step, which waited for the copies in, and the copies out
-  join.done = true;
+  CKR(cudaStreamSynchronize(st));
   float gemm_ms = 0, all_ms = 0;
-  for (int c = 0; c < K; ++c) {   // the steps' products (their waits for copies are between them)
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->events[3 * c + 1], ctx->events[3 * c + 2]);
-    gemm_ms += ms;
-  }
+  cudaEventElapsedTime(&gemm_ms, ctx->ev[0], ctx->ev[1]);
   cudaEventElapsedTime(&all_ms, ctx->ev[5], ctx->ev[2]);
   ctx->stats.renorm_ms = gemm_ms;
   ctx->stats.renorm_e2e_ms = all_ms;

@@ -102,9 +102,9 @@ constexpr int BM = 64, BN = 64;
 // Tiling and scheduling choices the autotuner searches (defaults: the values
 // set by hand for the 4x24 m = 2000 superblock).
 struct TuneParams {
-  int items_per_cta = 6;    // FP64: split-K aims at this many items per resident CTA ...
+  int items_per_cta = 6;    // FP64: split-K aims at this many items per CTA of ctas_per_sm ...
   int min_ksteps = 256;     // ... never cutting an item below this many inner-dimension steps
-  int ctas_per_sm = 4;      // FP64: resident CTAs per SM of the grouped kernel (1..4)
+  int ctas_per_sm = 4;      // FP64: CTAs per SM that items are cut for; two (or one) are resident
   int oz_bn = 0;            // split precision: N tile (0: the default of the slice count)
   int oz_item_cost = 4;     // split precision: per-item cost, in k-blocks, of the static schedule
   bool operator==(const TuneParams &o) const {

@@ -6,7 +6,7 @@
 // context's precision mode; a candidate replaces the current best when it is
 // at least 2 % faster (so that timing noise does not move the choice).
 //   FP64            items_per_cta {3, 6, 12}, min_ksteps {128, 256, 512},
-//                   ctas_per_sm {2, 3, 4}
+//                   ctas_per_sm {2, 3, 4} (the count that items are cut for)
 //   split precision oz_bn {48, 32} (5 slices), oz_item_cost {2, 4, 8}
 #include <cuda_runtime.h>
 
