@@ -477,8 +477,8 @@ int tj_model_wave_multi(tj_ctx *ctx, int n, const tj_lattice *const *lat, const 
 
 /* ------------------------------------------------------------ autotuning */
 /* No counterpart in the reference.  The tiling of the grouped FP64 GEMM
- * (split-K granularity: items per resident CTA and minimum inner-dimension
- * steps per item; resident CTAs per SM) and of the split-precision GEMM (N
+ * (split-K granularity: items per CTA, CTAs per SM that they are cut for and
+ * minimum inner-dimension steps per item) and of the split-precision GEMM (N
  * tile, per-item cost of its static schedule) is chosen per block-size
  * histogram of the H*psi plan -- its GEMM tasks counted by (log2 M, log2 N,
  * log2 K) -- by timing H*psi with each candidate (coordinate descent from the
