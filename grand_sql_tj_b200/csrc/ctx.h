@@ -76,7 +76,7 @@ struct tj_ctx {
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t tev[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};   // truncation stages
   int prec_mode = TJ_PREC_FP64, slices = 6;
-  double wait_s = 2.0;        // limit of the split-precision GEMM's pipeline waits (tj_set_wait_limit)
+  double wait_s = 2.0;        // limit of the kernels' waits for one another's copies (tj_set_wait_limit)
   // tiling / schedule choices in use, and how they are chosen (TJ_TUNE_*)
   tjb::TuneParams tune;
   int autotune = TJ_TUNE_CACHED;

@@ -418,7 +418,7 @@ __device__ __forceinline__ double block_sum1(double x, double *red, int &half) {
 constexpr int TD_NB = 16;              // reflectors of a panel
 constexpr int TD_LD = 2 * TD_NB + 2;   // row of V and W in shared memory: V, W, pad
 constexpr int TD_PT = 3 * TD_NB;       // a CTA's parts: W^T a, V^T a, a.(A a) by warp
-constexpr long long TD_WAIT = 4000000000LL;   // cycles until a wait for the other CTAs' stores gives up
+constexpr double TD_CYCLES = 2e9;      // cycles a second, for the limit of the waits (tj_set_wait_limit)
 constexpr int TD_PL = TD_PT + 1;       // their stride: odd, so that the CTAs' parts lie in different banks
 
 // Doubles of shared memory besides the resident columns.
@@ -471,8 +471,20 @@ __device__ __forceinline__ void td_send(uint32_t dst, double v, uint32_t bar) {
 __device__ __forceinline__ void td_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase of the given parity; false if it does not come (TD_WAIT).
-__device__ __forceinline__ bool td_wait(uint32_t bar, uint32_t parity) {
+// Waits for the phase of the given parity; false if it does not come within
+// `limit` cycles (0: unless it has come already).
+__device__ __forceinline__ bool td_wait(uint32_t bar, uint32_t parity, long long limit) {
+  if (limit <= 0) {   // try_wait may block for a while, test_wait does not
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+  }
   const long long c0 = clock64();
   do {
     uint32_t ok;
@@ -484,7 +496,7 @@ __device__ __forceinline__ bool td_wait(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-  } while (clock64() - c0 < TD_WAIT);
+  } while (clock64() - c0 < limit);
   return false;
 }
 __device__ __forceinline__ void td_dmma(double (&c)[2], double a, double b) {
@@ -497,7 +509,7 @@ template <int CL>
 __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aall, const int64_t *off,
                              const int *dims, const int64_t *eoff, double *dall, double *eall, double *tauall,
                              double *Wall, double *info, double *dsall, double *e2all, double *sm, int64_t smem_doubles,
-                             double *red, uint64_t *mbar, int *status) {
+                             double *red, uint64_t *mbar, int *status, long long limit) {
   constexpr int NB = TD_NB, NW = EIG_THREADS / 32, MW = NW - 1;   // MW warps multiply, the last finds the scale
   static_assert(NB == 16 && NW == 16 && CL <= NW, "the warps' shares below");
   const int n = dims[s], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -536,7 +548,17 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  bool late = false;   // a wait has given up: the rest runs through without waiting
+  // A wait that gives up leaves its phase open.  The thread that gave up neither
+  // sends nor arrives nor waits any more; it only runs through the rest of the
+  // steps, whose barriers the others count on, and the result is not used.  So
+  // every store and every arrival is of a thread that has seen all earlier
+  // phases complete, as the order above asks; and whoever misses the stores (or
+  // its thread 0's arrival) gives up at its own next wait, so that no mbarrier
+  // meets more than two steps' bytes.
+  bool late = false;
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (!late) late = !td_wait(bar, parity, limit);
+  };
   int p = 0;   // the panel's first column
   // the panel's V (below each reflector's first row), d, e and tau to global memory
   auto flush = [&](int cols) {
@@ -717,12 +739,12 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
       __syncthreads();
     }
     // warp w sends the owned entries to CTA w
-    if (warp < CL && warp != rank) {
+    if (!late && warp < CL && warp != rank) {
       const uint32_t o = td_remote(td_smem(me), warp), ob = td_remote(bar0, warp);
       for (int q = q0 + lane; q < nq; q += 32) td_send(o + q * 8, me[q], ob);
     }
-    if (tid == 0) td_expect(bar0, (uint32_t)(n - k - (nq - q0)) * 8);
-    if (!late) late = !td_wait(bar0, k & 1);
+    if (!late && tid == 0) td_expect(bar0, (uint32_t)(n - k - (nq - q0)) * 8);
+    wait(bar0, k & 1);
     if (rank == 0 && tid == 0) de[jc] = col[k % CL * lc + k / CL];
     if (k == n - 1) break;
     // ---- the reflector's scale; A a
@@ -809,7 +831,7 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     }
     __syncthreads();
     // warp w sends the parts, and the owner of row k1 its row, to CTA w
-    if (warp < CL) {
+    if (!late && warp < CL) {
       const uint32_t o = td_remote(td_smem(part + rank * TD_PL), warp), ob = td_remote(bar1, warp);
       td_send(o + lane * 8, stg[lane], ob);
       if (lane < NB) td_send(o + (2 * NB + lane) * 8, stg[2 * NB + lane], ob);
@@ -819,8 +841,8 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
         if (lane < 2) td_send(b + (2 * NB + lane) * 8, (lane ? rk : ys)[k1 / CL], ob);
       }
     }
-    if (tid == 0) td_expect(bar1, (CL * TD_PT + TD_LD) * 8);
-    if (!late) late = !td_wait(bar1, k & 1);
+    if (!late && tid == 0) td_expect(bar1, (CL * TD_PT + TD_LD) * 8);
+    wait(bar1, k & 1);
   }
   __syncthreads();
   flush(n - 1 - p);
@@ -828,15 +850,16 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     d[n - 1] = de[n - 1 - p];
     tau[n - 1] = 0.0;
   }
-  if (__syncthreads_or(late)) {
-    // what was not waited for may still be on its way: no CTA leaves at once
-    if (tid == 0) atomicOr(status, 4);
+  late = __syncthreads_or(late);
+  if (late && tid == 0) atomicOr(status, 4);
+  __threadfence();
+  cl.sync();   // every owner's writes are visible, and no CTA sends any more
+  if (late) {
+    // what this CTA did not wait for may still be on its way here: it does not leave at once
     const long long c0 = clock64();
     while (clock64() - c0 < 1000000) {
     }
   }
-  __threadfence();
-  cl.sync();   // every owner's writes are visible
   if (rank == 0) tridiag_info(s, n, d, e, info, dsall + eoff[s], e2all + eoff[s], red);
 }
 
@@ -849,7 +872,7 @@ template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
     tridiag_kernel(double *Aall, const int64_t *off, const int *dims, const int64_t *eoff, const int *tsec,
                    const int *tbig, double *dall, double *eall, double *tauall, double *Wall, double *info,
-                   double *dsall, double *e2all, int64_t smem_doubles, int *status) {
+                   double *dsall, double *e2all, int64_t smem_doubles, int *status, long long limit) {
   extern __shared__ __align__(16) double td_sm[];
   __shared__ double red[48];
   __shared__ double sh_tau, sh_scl;
@@ -859,7 +882,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(EIG_THREADS)
   const int s = tsec[blockIdx.x];
   if (tbig[b]) {
     tridiag_coop<CL>(cl, rank, s, Aall, off, dims, eoff, dall, eall, tauall, Wall, info, dsall, e2all, td_sm, smem_doubles,
-                     red, mbar, status);
+                     red, mbar, status, limit);
   } else if (s >= 0 && dims[s] > 0) {
     const int n = dims[s];
     if (n <= 32)
@@ -1937,16 +1960,17 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     // tridiagonal reduction, then all eigenvalues
     if (nclus) {
       const int *d_tsec = (const int *)(tbase + p_tsec), *d_tbig = (const int *)(tbase + p_tbig);
+      const long long wait_cycles = (long long)(ctx->wait_s * TD_CYCLES);
       if (tcl == 16) {
         CKT(cudaFuncSetAttribute(tridiag_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<16><<<nclus * 16, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
                                                                  dd, de, dtau, ctx->trB.d() + rlen, dinfo, dds, de2, (int64_t)(tsm / 8),
-        d_status);
+        d_status, wait_cycles);
       } else {
         CKT(cudaFuncSetAttribute(tridiag_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
         tridiag_kernel<8><<<nclus * 8, EIG_THREADS, tsm, st>>>(ctx->trB.d(), d_roff, d_dims, d_eoff, d_tsec, d_tbig,
                                                                dd, de, dtau, ctx->trB.d() + rlen, dinfo, dds, de2, (int64_t)(tsm / 8),
-        d_status);
+        d_status, wait_cycles);
       }
       CKT(cudaGetLastError());
     }

@@ -158,7 +158,9 @@ int tj_set_precision(tj_ctx *ctx, int mode, int slices);
  * metadata) gives up after `seconds` (default 2): the kernel then lets its
  * other roles stop, waits for its copies and MMAs in flight (with their own
  * 2 s bound), releases its tensor memory and returns, and the call returns
- * TJ_ERR_TIMEOUT; the context stays usable.  seconds in [0, 60]. */
+ * TJ_ERR_TIMEOUT; the context stays usable.  The same limit holds for the
+ * waits of the truncation's tridiagonal reduction by a cluster of CTAs for one
+ * another's data.  seconds in [0, 60]. */
 int tj_set_wait_limit(tj_ctx *ctx, double seconds);
 /* Invalidates the operators and task lists cached for the current DMRG step. */
 int tj_step_begin(tj_ctx *ctx);
