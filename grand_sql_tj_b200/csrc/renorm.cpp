@@ -752,14 +752,34 @@ uint64_t key_block(uint64_t h, const tj_block &b) {
   if (b.num > 0 && b.sub) h = key_bytes(h, b.sub, sizeof(tj_block_sub) * b.num);
   return h;
 }
-// structural key of a renormalisation call: tables and data pointers (the
-// two calls of the result protocol must pass the same inputs)
+// n entries of a table; nothing of one that is missing or has no entries (the
+// plan compiler refuses such a call)
+template <class T>
+uint64_t key_table(uint64_t h, const T *p, int64_t n) {
+  return p && n > 0 ? key_bytes(h, p, sizeof(T) * (size_t)n) : h;
+}
+// Key of all that a compiled renormalisation holds of its inputs: the tables
+// themselves, with the couplings and site energies that are coefficients of its
+// work list, and the places of the operators' arrays (whose values are read at
+// each call).
 uint64_t renorm_key(const tj_lattice *lat, int side, int mshift, const tj_model *pre, const tj_basis *basis,
                     const tj_block *trun) {
   uint64_t h = 1469598103934665603ull;
   h = key_bytes(h, lat, sizeof *lat);
   h = key_bytes(h, &side, sizeof side);
   h = key_bytes(h, &mshift, sizeof mshift);
+  const int64_t ns = lat->num_site, ns1 = ns + 1;
+  h = key_table(h, lat->neib, ns1 * lat->neibt);
+  h = key_table(h, lat->inb1, ns1 * ns1);
+  h = key_table(h, lat->nleg11, ns);
+  if (side == 1) {   // read for an environment only
+    h = key_table(h, lat->nposi_dm, ns1);
+    h = key_table(h, lat->nposi_lat, ns1);
+  }
+  h = key_table(h, lat->jt, ns1 * lat->neibt);
+  h = key_table(h, lat->jd, ns1 * lat->neibt);
+  h = key_table(h, lat->jn, lat->neibt);
+  h = key_table(h, lat->esite, ns1);
   h = key_bytes(h, pre, sizeof *pre);
   h = key_block(h, pre->ham);
   for (int i = 0; i < pre->nsub && pre->sub; ++i) {
@@ -767,7 +787,11 @@ uint64_t renorm_key(const tj_lattice *lat, int side, int mshift, const tj_model 
     h = key_block(key_block(key_block(key_block(h, s.elec_up), s.elec_down), s.spin_sd), s.num_sn);
   }
   h = key_bytes(h, basis, sizeof *basis);
-  if (basis->sub) h = key_bytes(h, basis->sub, sizeof(tj_basis_map) * basis->num);
+  h = key_table(h, basis->sub, basis->num);
+  int64_t nm = 0;
+  for (int i = 0; i < basis->num && basis->sub; ++i)
+    nm = std::max(nm, (int64_t)basis->sub[i].first + basis->sub[i].num);
+  h = key_table(h, basis->maps, nm);
   return key_block(h, *trun);
 }
 

@@ -1,0 +1,68 @@
+"""Inputs changed in place between two calls, the arrays and their tables staying
+where they are: the later call gives the result of the new values.
+
+  * tj_get_hamiltonian: couplings, site energies and the places of a basis's
+    states, against the oracle on the same inputs (<= 1e-12 of the largest entry).
+"""
+import ctypes as C
+import os
+
+import numpy as np
+import pytest
+
+from grand_sql_tj_b200 import synth
+from grand_sql_tj_b200.structs import Basis, BasisMap, call_model_result
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(product_lib):
+    from grand_sql_tj_b200.lib import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _data(m):
+    d = [sb.mat.reshape(-1, order="F") for b in [m.ham] + [getattr(s, k) for s in m.sub for k in
+                                                          ("elec_up", "elec_down", "spin_sd", "num_sn")] for sb in b.subs]
+    return np.concatenate(d)
+
+
+@pytest.mark.parametrize("side", [0, 1])
+@pytest.mark.parametrize("what", ["esite", "jt", "jd", "jn", "basis"])
+def test_renorm(ctx, oracle_lib, product_lib, what, side):
+    from oracle import oracle
+    oracle.set_threads(os.cpu_count() or 1)
+    rc = synth.renorm_case("cyl4", side=side)
+    pp, pb, pt = rc.pre.pack(), rc.basis.pack(), rc.trun.pack()
+
+    def call():
+        r, m = call_model_result(lambda res: product_lib.tj_get_hamiltonian(
+            ctx.h, C.byref(rc.lat.c), rc.side, rc.mshift, C.byref(pp.c), C.byref(pb.c), C.byref(pt.c), res))
+        assert r == 0
+        return _data(m)
+
+    first = call()
+    basis = rc.basis
+    if what == "basis":
+        # two equally large parts of each sector change places
+        maps = []
+        for i, m in enumerate(basis.maps):
+            subs = list(m.subs)
+            pair = [(a, b) for a in range(len(subs)) for b in range(a) if subs[a][1] == subs[b][1]][:1]
+            for a, b in pair:
+                subs[a], subs[b] = (subs[b][0],) + subs[a][1:], (subs[a][0],) + subs[b][1:]
+                ca, cb = pb.maps[pb.sub[i].first + a], pb.maps[pb.sub[i].first + b]
+                ca.spos, cb.spos = cb.spos, ca.spos
+            maps.append(BasisMap(m.new_num_up, m.new_num_down, subs))
+        basis = Basis(basis.len, maps)
+    else:
+        getattr(rc.lat, what)[:] *= 1.5
+        if what == "jn":
+            rc.lat.jn[:] += 0.25
+    second = call()
+    ref = _data(oracle.get_hamiltonian(rc.lat, rc.side, rc.mshift, rc.pre, basis, rc.trun))
+    assert np.max(np.abs(ref - first)) > 1e-6 * np.max(np.abs(ref))   # the change matters
+    assert np.max(np.abs(second - ref)) <= 1e-12 * np.max(np.abs(ref))
