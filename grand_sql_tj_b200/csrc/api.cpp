@@ -674,6 +674,10 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   if ((rc = run_hpsi(ctx, vec(1), Y, false))) return rc;
   dot_into(vec(1), Y, alpha + 1);
   double ritzmin = 0, hb = 0, hl = 0;
+  const int *err = ctx->oz ? (const int *)((char *)ctx->ozMisc.p + 64) : nullptr;   // error word of the split kernels
+  int *const err1 = (int *)(ctx->pinned + LZ_HOST * LZ_RING);   // its value after the first H*psi
+  *err1 = 0;
+  if (err) CK(cudaMemcpyAsync(err1, err, sizeof(int), cudaMemcpyDeviceToHost, st));
   if ((rc = fetch(alpha + 1, &ritzmin))) return rc;
   int last = 1;
   const int one = 1;
@@ -692,7 +696,6 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-  const int *err = ctx->oz ? (const int *)((char *)ctx->ozMisc.p + 64) : nullptr;
   if (is_short) {
     launch_lz_step_short(V, ld, itd, Y, X, D, S, st);
   } else {
@@ -729,9 +732,11 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   // known, and the Ritz value (one block) is found beside it on a second
   // stream (2x16 ladder m = 256: 77 us an iteration
   // with both in line, 57 so).  The iteration launched past the last is dropped as
-  // above, and its error flags with it: the flags are those published with the
-  // scalars.  A long vector's iteration costs more than all those gaps.
-  int flags = 0;
+  // above.  A long vector's iteration costs more than all those gaps.
+  // `flags` is the error word after the last H*psi that the result uses: as
+  // published with the scalars of each step that is kept (of a step that is
+  // dropped it may tell of the 0 / 0 of a vanishing beta).
+  int flags = *err1;
   int launched = 1;   // the step after the last one launched
   while (last < LOOP_IN) {
     for (; launched <= last + (is_short ? 1 : 0) && launched < LOOP_IN; ++launched) {
@@ -747,13 +752,13 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
     const double *seen = ctx->pinned + LZ_HOST * (last % LZ_RING);
     hb = seen[0];
     hl = seen[1];
-    flags = (int)seen[2];
     ++last;
     if (!std::isfinite(hb)) return set_err(TJ_ERR_NUMERIC, "Lanczos: non-finite beta");
     if (std::fabs(hb) <= lanzero) {
       --last;
       break;
     }
+    flags = (int)seen[2];
     if (!std::isfinite(hl)) return set_err(TJ_ERR_NUMERIC, "Lanczos: non-finite Ritz value");
     if (std::fabs(hl - ritzmin) <= lanzero || last == LOOP_IN) {
       ritzmin = hl;
