@@ -325,11 +325,14 @@ extern "C" int tj_wave_trans(tj_ctx *ctx, int direction, const tj_basis *sys_bs,
   CKW(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   // The old wavefunction goes up while the plan is made (280 and 150 us on the
-  // 4x24 m = 2000 superblock, one after the other before).
+  // 4x24 m = 2000 superblock, one after the other before).  The device time is
+  // that from this copy's start to the end (events 5 and 2), without the time
+  // between the copy and the plan's end (3 and 4) where the plan takes longer.
   if ((rc = ctx->wtOld.reserve(sizeof(double) * (old_wave->dim + 4)))) return rc;
   CKW(cudaEventRecord(ctx->ev[5], st));
   const bool ahead = old_wave->num > 0;   // without sectors there may be no array: the plan decides first
   if (ahead) CKW(upload(ctx, ctx->wtOld.d(), old_wave->data, old_wave->dim, st));
+  CKW(cudaEventRecord(ctx->ev[3], st));
   HpsiPlan P;
   std::string msg;
   const auto t0 = std::chrono::steady_clock::now();
@@ -346,6 +349,9 @@ extern "C" int tj_wave_trans(tj_ctx *ctx, int direction, const tj_basis *sys_bs,
     cudaStreamSynchronize(st);
     return rc;
   }
+  const bool idle = cudaEventQuery(ctx->ev[3]) == cudaSuccess;
+  if (!idle) cudaGetLastError();   // "not ready" is no error
+  if (idle) CKW(cudaEventRecord(ctx->ev[4], st));
   if (!ahead) CKW(upload(ctx, ctx->wtOld.d(), old_wave->data, old_wave->dim, st));
   for (const auto &u : P.uploads)
     if (u.n > 0) CKW(upload(ctx, ctx->wtOps.d() + u.dst, u.src, u.n, st));
@@ -407,10 +413,11 @@ extern "C" int tj_wave_trans(tj_ctx *ctx, int direction, const tj_basis *sys_bs,
     int rc = download(ctx, new_wave->data, ctx->wtNew.d(), D, st);
     if (!rc) rc = res_keep(ctx, new_wave->data, D, ctx->wtNew.d(), st);
     if (rc) return rc;
-    float ms = 0;
+    float ms = 0, idle_ms = 0;
     if (cudaEventRecord(ctx->ev[2], st) == cudaSuccess && cudaEventSynchronize(ctx->ev[2]) == cudaSuccess &&
-        cudaEventElapsedTime(&ms, ctx->ev[5], ctx->ev[2]) == cudaSuccess)
-      ctx->stats.wt_ms = ms;
+        cudaEventElapsedTime(&ms, ctx->ev[5], ctx->ev[2]) == cudaSuccess &&
+        (!idle || cudaEventElapsedTime(&idle_ms, ctx->ev[3], ctx->ev[4]) == cudaSuccess))
+      ctx->stats.wt_ms = ms - idle_ms;
     cudaGetLastError();
   }
   if (!(h_nrm > 0.0) || !std::isfinite(h_nrm))
