@@ -1253,7 +1253,10 @@ static int meas_call(tj_ctx *ctx, uint64_t key, tj_block_result *out,
   CKR(cudaSetDevice(ctx->device));
   if (!ctx->meas) ctx->meas = new_meas_state();
   LastOp &L = ctx->meas->last;
-  if (!(L.valid && L.key == key)) {
+  // The key holds addresses, so a result answers one pair of calls only: the
+  // second, with the caller's arrays, after a first without them.
+  const bool second = out->subs && out->data;
+  if (!(second && L.valid && L.key == key)) {
     L.valid = false;
     std::string msg;
     int rc;
@@ -1267,7 +1270,9 @@ static int meas_call(tj_ctx *ctx, uint64_t key, tj_block_result *out,
     L.key = key;
     L.valid = true;
   }
-  return finish(ctx, L.op, out);
+  const int rc = finish(ctx, L.op, out);
+  if (second && rc == TJ_OK) L.valid = false;
+  return rc;
 }
 
 extern "C" int tj_get_oper(tj_ctx *ctx, int side, int dia, const tj_chain *chain, const tj_block *st_oper, int old_idx,

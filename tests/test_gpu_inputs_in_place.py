@@ -2,7 +2,9 @@
 where they are: the later call gives the result of the new values.
 
   * tj_get_hamiltonian: couplings, site energies and the places of a basis's
-    states, against the oracle on the same inputs (<= 1e-12 of the largest entry).
+    states, against the oracle on the same inputs (<= 1e-12 of the largest entry);
+  * tj_update_trun (a measurement operator's step): the operator doubled, so
+    exactly twice the result.
 """
 import ctypes as C
 import os
@@ -11,7 +13,7 @@ import numpy as np
 import pytest
 
 from grand_sql_tj_b200 import synth
-from grand_sql_tj_b200.structs import Basis, BasisMap, call_model_result
+from grand_sql_tj_b200.structs import Basis, BasisMap, TjBlockResult, call_block_result, call_model_result
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +68,25 @@ def test_renorm(ctx, oracle_lib, product_lib, what, side):
     ref = _data(oracle.get_hamiltonian(rc.lat, rc.side, rc.mshift, rc.pre, basis, rc.trun))
     assert np.max(np.abs(ref - first)) > 1e-6 * np.max(np.abs(ref))   # the change matters
     assert np.max(np.abs(second - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_measurement_operator(ctx, product_lib):
+    rc = synth.renorm_case("cyl4", side=0)
+    ori, trun = rc.pre.ham, synth.random_trun(
+        Basis(rc.pre.len, [BasisMap(s.num_up, s.num_down, [(0, s.mat.shape[0], 0, 0, 0, 0)]) for s in rc.pre.ham.subs]),
+        30, np.random.default_rng(3))
+    po, pt = ori.pack(), trun.pack()
+
+    def call():
+        r, b = call_block_result(lambda res: product_lib.tj_update_trun(ctx.h, 1, C.byref(po.c), C.byref(pt.c), res))
+        assert r == 0
+        return np.concatenate([s.mat.reshape(-1, order="F") for s in b.subs])
+
+    first = call()
+    po.data *= 2.0
+    assert np.max(np.abs(first)) > 0 and np.array_equal(call(), 2.0 * first)
+    # a first call that no second followed
+    res = TjBlockResult()
+    assert product_lib.tj_update_trun(ctx.h, 1, C.byref(po.c), C.byref(pt.c), C.byref(res)) == 0
+    po.data *= 2.0
+    assert np.array_equal(call(), 4.0 * first)
