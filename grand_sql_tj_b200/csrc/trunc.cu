@@ -1818,7 +1818,11 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
   }
   const uint64_t h = hash_data(wave->data, D);
   TruncCache &tc = g_tc;
-  const bool hit = tc.valid && tc.data == wave->data && tc.dim == D && tc.side == side && tc.kept_min == kept_min &&
+  // The kept operator answers one pair of calls only, the second (with the
+  // caller's arrays) after a first without them: the fingerprint is of samples,
+  // and psi may have changed in place since.
+  const bool second = out->sub && out->data;
+  const bool hit = second && tc.valid && tc.data == wave->data && tc.dim == D && tc.side == side && tc.kept_min == kept_min &&
                    tc.kept_max == kept_max && tc.trun_err == trun_err && tc.hash == h && tc.ctx == ctx &&
                    tc.seq == ctx->trunc_seq;
   if (!hit) {
@@ -2344,6 +2348,7 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       const int rc = res_keep(ctx, udata, tc.len, tc.dev, ctx->stream);
       if (rc) return rc;
     }
+    tc.valid = false;
   }
   return TJ_OK;
 }

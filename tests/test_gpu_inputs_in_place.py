@@ -4,7 +4,9 @@ where they are: the later call gives the result of the new values.
   * tj_get_hamiltonian: couplings, site energies and the places of a basis's
     states, against the oracle on the same inputs (<= 1e-12 of the largest entry);
   * tj_update_trun (a measurement operator's step): the operator doubled, so
-    exactly twice the result.
+    exactly twice the result;
+  * tj_truncation: entries of the wavefunction changed, against the same values
+    in another array (the same bits).
 """
 import ctypes as C
 import os
@@ -13,7 +15,7 @@ import numpy as np
 import pytest
 
 from grand_sql_tj_b200 import synth
-from grand_sql_tj_b200.structs import Basis, BasisMap, TjBlockResult, call_block_result, call_model_result
+from grand_sql_tj_b200.structs import Basis, BasisMap, TjBlockResult, Wave, WaveSector, call_block_result, call_model_result
 
 pytestmark = pytest.mark.gpu
 
@@ -90,3 +92,17 @@ def test_measurement_operator(ctx, product_lib):
     assert product_lib.tj_update_trun(ctx.h, 1, C.byref(po.c), C.byref(pt.c), C.byref(res)) == 0
     po.data *= 2.0
     assert np.array_equal(call(), 4.0 * first)
+
+
+def test_truncation(ctx):
+    rng = np.random.default_rng(7)
+    n = 90
+    w = Wave(3, 3, [WaveSector(4, 0, 4, 0, n, n)], rng.standard_normal(n * n))
+    for at in range(4000, 4006):   # one entry at a time
+        _, b = ctx.truncation(w, 0, 20, 20, 0.0)
+        before = b.subs[0].mat.copy()
+        w.data[at] += 0.5
+        _, got = ctx.truncation(w, 0, 20, 20, 0.0)
+        _, ref = ctx.truncation(w.copy(), 0, 20, 20, 0.0)
+        assert np.array_equal(got.subs[0].mat, ref.subs[0].mat)
+        assert not np.array_equal(got.subs[0].mat, before)
