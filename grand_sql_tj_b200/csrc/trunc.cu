@@ -11,7 +11,7 @@
 // eigen-decomposition follows the direct route of DSYEV's first stage and
 // replaces its second: every sector is reduced to tridiagonal form by
 // Householder reflections (one CTA per sector, or a thread-block cluster of
-// 8-16 CTAs for sectors of 320 states and more), all eigenvalues come from
+// 16 (8) CTAs for a large one), all eigenvalues come from
 // Sturm-count multisection (one warp per eigenvalue), the host selects the
 // kept states exactly as den_mat.f90 does, and only the kept eigenvectors
 // are computed: inverse iteration on the tridiagonal matrix (one thread per
@@ -48,11 +48,15 @@ constexpr double EIG_SAFMIN = 2.2250738585072014e-308;   // smallest normal FP64
 constexpr int ORTH_THREADS = 512;
 // A sector of up to TD_SMALL states is reduced in one CTA's shared memory (62
 // states: 87 us, 133 from L2; with three rows a lane 96 would take 248 and 238,
-// with five 160 720 and 558), one of at least TD_BIG by a whole cluster: alone, 191 states
-// take 0.84 ms in one CTA, 192 take 0.54 in a cluster, 261 1.77 and 0.75, 319 2.98
-// and 0.95; but only seven clusters of 16 run at a time, so the line lies above
-// the break-even of one sector (14 sectors of 180: 0.74 ms and 1.01).
-constexpr int TD_SMALL = 64, TD_BIG = 192;
+// with five 160 720 and 558), one of up to TD_ONE states by one CTA from L2, one
+// of at least TD_BIG by a whole cluster, and those between by either, whichever
+// is done first for all sectors of a call (td_by_cluster).  Alone, 191 states
+// take 0.85 ms in one CTA, 192 take 0.54 in a cluster and 0.84 in one CTA, 260
+// 0.76 and 1.77, 319 0.96 and 3.0; but only seven clusters of 16 run at a time,
+// so many equal sectors are done sooner side by side (14 of 180 states: 0.74 ms
+// in one CTA each, 1.01 in clusters; 22 of 208: 1.03 and 2.32; 22 of 260: 1.78
+// and 2.96).
+constexpr int TD_SMALL = 64, TD_ONE = 191, TD_BIG = 320;
 
 // Sum of the warps' partial sums r[0..nw-1] by every warp: lane w takes
 // r[w] and a shuffle tree adds them, in the same order in every warp (a
@@ -1769,15 +1773,20 @@ struct Tables {
   size_t size() const { return buf.size() + extra; }
 };
 
-// Clusters of 16 CTAs (a non-portable size) where the GPU can schedule one
-// with `threads` threads and `smem` bytes of dynamic shared memory per CTA;
-// otherwise 8.  Asked once per kernel and shared-memory size.
+struct ClusterSize {
+  size_t smem;
+  int ctas;     // 16 (a non-portable size) or 8
+  int active;   // clusters of 16 that run at a time
+};
+// Clusters of 16 CTAs where the GPU can schedule one with `threads` threads and
+// `smem` bytes of dynamic shared memory per CTA; otherwise 8.  Asked once per
+// kernel and shared-memory size.
 template <typename K16>
-int cluster_size(K16 kernel16, int threads, size_t smem) {
-  static thread_local std::vector<std::pair<size_t, int>> seen;
+ClusterSize cluster_size(K16 kernel16, int threads, size_t smem) {
+  static thread_local std::vector<ClusterSize> seen;
   for (auto &x : seen)
-    if (x.first == smem) return x.second;
-  int cl = 8;
+    if (x.smem == smem) return x;
+  ClusterSize c{smem, 8, 0};
   if (cudaFuncSetAttribute(kernel16, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
       cudaFuncSetAttribute(kernel16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess) {
     cudaLaunchConfig_t cfg;
@@ -1793,11 +1802,49 @@ int cluster_size(K16 kernel16, int threads, size_t smem) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel16, &cfg) == cudaSuccess && n >= 1) cl = 16;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel16, &cfg) == cudaSuccess && n >= 1) {
+      c.ctas = 16;
+      c.active = n;
+    }
   }
   cudaGetLastError();
-  seen.push_back({smem, cl});
-  return cl;
+  seen.push_back(c);
+  return c;
+}
+
+// How many of the sectors (n: their states, largest first), the largest ones,
+// are reduced by a cluster of 16 CTAs each, the others one to a CTA, 16 to a
+// cluster: at least those of TD_BIG states, at most those above TD_ONE.  Where
+// they do not all run at a time (`active` clusters do, started in this order),
+// clusters give way to CTAs if the last sector is then done a tenth sooner.  The
+// times (us) fit those of one sector to 8 % from 130 states on: by a cluster
+// 0.54 ms (192 states), 0.96 (319), 1.27 (400), 4.1 (857), 12.1 (1400); by a CTA
+// 0.57 (160), 0.84 (192), 1.45 (240), 2.6 (300), and with the shared memory that
+// clusters ask for, which leaves it no L1, 1.12 (200), 1.65 (240), 2.9 (300).
+int td_by_cluster(const std::vector<int> &n, int active) {
+  const int ns = (int)n.size();
+  int lo = 0;
+  while (lo < ns && n[lo] >= TD_BIG) ++lo;
+  int hi = lo;
+  while (hi < ns && n[hi] > TD_ONE) ++hi;
+  if (hi == lo || active < 1 || hi + (ns - hi + 15) / 16 <= active) return hi;
+  auto done = [&](int b) {   // when the last cluster ends, b sectors having one each
+    std::vector<double> end(active, 0.0);
+    auto start = [&](double t) { *std::min_element(end.begin(), end.end()) += t; };
+    for (int i = 0; i < b; ++i) start(n[i] * (2.7 + 2.85e-6 * n[i] * n[i]));
+    for (int i = b; i < ns; i += 16) start(n[i] * ((b ? 2.45 : 1.45) + 7.95e-5 * n[i] * n[i]));
+    return *std::max_element(end.begin(), end.end());
+  };
+  int best = hi;
+  double t = 0.9 * done(hi);
+  for (int b = hi - 1; b >= lo; --b) {
+    const double tb = done(b);
+    if (tb < t) {
+      t = tb;
+      best = b;
+    }
+  }
+  return best;
 }
 
 }  // namespace
@@ -1896,37 +1943,47 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
     double *dd = ctx->trD.d(), *de = dd + etot, *dtau = de + etot, *dev = dtau + etot, *dds = dev + etot,
            *de2 = dds + etot, *dinfo = de2 + etot;
     // clusters of the tridiagonal reduction: one per large sector, then the
-    // small sectors tcl at a time (largest first)
+    // others tcl at a time (largest first)
+    while (!order.empty() && dims[order.back()] == 0) order.pop_back();
+    std::vector<int> sizes;
+    for (int x : order) sizes.push_back(dims[x]);
     // shared memory: a small sector's matrix, a middle one's vectors; for one
     // reduced by a cluster as much as a CTA may have (its columns)
-    size_t tsm = 0;
-    for (int n : dims)
-      if (n < TD_BIG)
-        tsm = std::max(tsm, sizeof(double) * (n <= TD_SMALL ? (size_t)n * (n + 2) : 3 * (size_t)n + EIG_THREADS));
-    if (maxn >= TD_BIG) {
-      tsm = std::max(tsm, sizeof(double) * (size_t)td_coop_doubles(maxn, 8));
-      int optin = 0;
-      cudaFuncAttributes fa;
-      if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
-          cudaFuncGetAttributes(&fa, tridiag_kernel<16>) == cudaSuccess && optin > (int)fa.sharedSizeBytes + 1024)
-        tsm = std::max(tsm, (size_t)(optin - (int)fa.sharedSizeBytes - 1024) / 256 * 256);
-      cudaGetLastError();
+    auto td_smem_bytes = [&](int big) {
+      size_t b = 0;
+      for (size_t q = big; q < sizes.size(); ++q) {
+        const size_t n = sizes[q];
+        b = std::max(b, sizeof(double) * (n <= TD_SMALL ? n * (n + 2) : 3 * n + EIG_THREADS));
+      }
+      if (big) {
+        b = std::max(b, sizeof(double) * (size_t)td_coop_doubles(maxn, 8));
+        int optin = 0;
+        cudaFuncAttributes fa;
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+            cudaFuncGetAttributes(&fa, tridiag_kernel<16>) == cudaSuccess && optin > (int)fa.sharedSizeBytes + 1024)
+          b = std::max(b, (size_t)(optin - (int)fa.sharedSizeBytes - 1024) / 256 * 256);
+        cudaGetLastError();
+      }
+      return b;
+    };
+    int nbig = 0;
+    while (nbig < (int)sizes.size() && sizes[nbig] > TD_ONE) ++nbig;
+    size_t tsm = td_smem_bytes(nbig);
+    ClusterSize tcs = cluster_size(tridiag_kernel<16>, EIG_THREADS, tsm);
+    if (tcs.ctas == 16) {
+      nbig = td_by_cluster(sizes, tcs.active);
+      tsm = td_smem_bytes(nbig);
+      tcs = cluster_size(tridiag_kernel<16>, EIG_THREADS, tsm);
     }
-    const int tcl = cluster_size(tridiag_kernel<16>, EIG_THREADS, tsm);
+    const int tcl = tcs.ctas;
     std::vector<int> tsec, tbig;
-    {
-      size_t q = 0;
-      for (; q < order.size() && dims[order[q]] >= TD_BIG; ++q) {
-        tsec.insert(tsec.end(), tcl, order[q]);
-        tbig.push_back(1);
-      }
-      std::vector<int> small;
-      for (; q < order.size(); ++q)
-        if (dims[order[q]] > 0) small.push_back(order[q]);
-      for (size_t i = 0; i < small.size(); i += tcl) {
-        for (int r = 0; r < tcl; ++r) tsec.push_back(i + r < small.size() ? small[i + r] : -1);
-        tbig.push_back(0);
-      }
+    for (int q = 0; q < nbig; ++q) {
+      tsec.insert(tsec.end(), tcl, order[q]);
+      tbig.push_back(1);
+    }
+    for (size_t i = nbig; i < order.size(); i += tcl) {
+      for (int r = 0; r < tcl; ++r) tsec.push_back(i + r < order.size() ? order[i + r] : -1);
+      tbig.push_back(0);
     }
     const int nclus = (int)tbig.size();
     // the small tables in one buffer and one copy
@@ -2173,7 +2230,7 @@ extern "C" int tj_truncation(tj_ctx *ctx, const tj_wave *wave, int side, int kep
       // clusters of the orthonormalisation: one per large kept block (cnt^2 n
       // above 3e7), then the other blocks ocl at a time, largest first
       const size_t osm = sizeof(double) * (3 * (size_t)maxn + (maxn + 7) / 8 + 8 + ORTH_THREADS);
-      const int ocl = cluster_size(orthonormalize_kernel<16>, ORTH_THREADS, osm);
+      const int ocl = cluster_size(orthonormalize_kernel<16>, ORTH_THREADS, osm).ctas;
       std::vector<int> oblk, obig;
       {
         std::vector<int> bo(ngrp);
