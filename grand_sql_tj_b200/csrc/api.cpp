@@ -689,7 +689,7 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   // next vector when |beta| <= lanzero; here that vector and its H*psi are
   // computed speculatively and dropped, with `last` restored, so the result
   // is the same.
-  auto ref = [&](int off) { return LzRef{V, ld, itd, off, nullptr}; };
+  auto ref = [&](int off) { return LzRef{V, ld, itd, off}; };
   const bool is_short = lz_short(D);
   cudaStream_t side = nullptr;
   if (is_short && (rc = ctx->side_stream(side))) return rc;
@@ -770,7 +770,7 @@ extern "C" int tj_lanczos_memo_new(tj_ctx *ctx, const tj_lattice *lat, const tj_
   // label 411: dstev('V') and the Ritz vector
   launch_tridiag_min(alpha + 1, beta + 1, last, lam, dz, 1, ctx->stream);
   if ((rc = ctx->vout.reserve(sizeof(double) * (D + 4)))) return rc;
-  launch_combine(V, ld, last, dz, ctx->vout.d(), D, 1, ctx->stream);
+  launch_combine(V, ld, last, dz, ctx->vout.d(), D, ctx->stream);
   norm_into(ctx->vout.d(), nrm);
   launch_scale_inv(ctx->vout.d(), nrm, D, ctx->stream);
   CK(cudaGetLastError());

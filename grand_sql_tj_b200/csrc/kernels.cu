@@ -556,19 +556,18 @@ void launch_scale_inv(double *x, const double *nrm, int64_t n, cudaStream_t s) {
 }
 
 __global__ void combine_kernel(const double *__restrict__ V, int64_t ld, int k, const double *__restrict__ coef,
-                               double *w, int64_t n, int assign) {
+                               double *w, int64_t n) {
   __shared__ double c[128];
   for (int j = threadIdx.x; j < k && j < 128; j += blockDim.x) c[j] = coef[j];
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double t = 0.0;
     for (int j = 0; j < k; ++j) t = t + c[j] * V[(int64_t)j * ld + i];
-    w[i] = assign ? t : w[i] - t;
+    w[i] = t;
   }
 }
-void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, int assign,
-                    cudaStream_t s) {
-  combine_kernel<<<vgrid(n), VT, 0, s>>>(V, ld, k, coef, w, n, assign);
+void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, cudaStream_t s) {
+  combine_kernel<<<vgrid(n), VT, 0, s>>>(V, ld, k, coef, w, n);
 }
 
 // Ordered integer image of a double: monotone in the value, with +0 and -0
@@ -775,7 +774,7 @@ void launch_tridiag_min(const double *a, const double *b, int n, double *lam, do
 // last block to finish adds the block partials in a fixed order, so the
 // result does not depend on the order the blocks run in.
 __device__ __forceinline__ double *lz_ptr(const LzRef &r) {
-  return r.fixed ? r.fixed : r.V + (int64_t)(*r.it + r.off - 1) * r.ld;
+  return r.V + (int64_t)(*r.it + r.off - 1) * r.ld;
 }
 
 // The block partial s (valid in thread 0) to partials[blockIdx.x]; the last
@@ -1185,9 +1184,9 @@ void launch_lz_publish_short(double *S, int L, double *host, cudaStream_t s) {
   lz_publish_short_kernel<<<1, TRI_THREADS, 0, s>>>(S, L, host);
 }
 
-// the elementwise kernels with a fused norm run on the grid of a dot product
-// (fewer partials for the last block to add); the Gram-Schmidt combination,
-// which streams L vectors per element, on the wider vector grid
+// partial sums a kernel may leave: the scaling and the dot product run on the
+// grid of a dot product (fewer partials for the last block to add), the
+// Gram-Schmidt kernels, which stream L vectors per element, on the slices
 int lz_blocks(int64_t n) { return std::max(lz_slices(n), dot_blocks(n)); }
 void launch_lz_update_gram_schmidt(const double *V, int64_t ld, const int *it, LzRef w, const double *src, int64_t n,
                                    double *S, double *mpartials, int kmax, const double *uu, double *coef,

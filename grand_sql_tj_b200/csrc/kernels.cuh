@@ -39,21 +39,19 @@ void launch_sum(const double *partials, int nblk, double *res, int sqrt_flag, cu
 int dot_blocks(int64_t n);
 // x = x / (*nrm)
 void launch_scale_inv(double *x, const double *nrm, int64_t n, cudaStream_t s);
-// w = w - sum_j coef[j] * V[j]    (or w = sum_j coef[j] V[j] when assign)
-void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, int assign,
-                    cudaStream_t s);
+// w = sum_j coef[j] V[j]
+void launch_combine(const double *V, int64_t ld, int k, const double *coef, double *w, int64_t n, cudaStream_t s);
 // lowest eigenvalue (and its eigenvector if vec) of the symmetric tridiagonal (a[0..n-1], b[0..n-2])
 void launch_tridiag_min(const double *a, const double *b, int n, double *lam, double *vec, int want_vec,
                         cudaStream_t s);
 
 // ---- Lanczos iteration with the step L read from device memory (*it) ----
-// A vector chosen when the kernel runs: vec(*it + off) = V + (*it + off - 1) * ld, or `fixed`.
+// A vector chosen when the kernel runs: vec(*it + off) = V + (*it + off - 1) * ld.
 struct LzRef {
   double *V;
   int64_t ld;
   const int *it;
   int off;
-  double *fixed;
 };
 // S: alpha(j) at S[j], beta(j) at S[128 + j], uu(j) at S[256 + j], the Ritz
 // value at S[512], a norm at S[513]; cnt: a zeroed int the kernels that end in
