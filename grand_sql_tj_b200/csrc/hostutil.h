@@ -11,7 +11,8 @@ namespace tjb {
 // Key of n bytes, chained onto h: 8 bytes a step in four independent lanes (a
 // byte at a time, the tables of one H*psi call took 390 us of its 1.26 ms in
 // split precision on the 4x24 m = 2000 superblock, now 15).  Every step is a
-// bijection of its lane for given input.
+// bijection of its lane for given input: an xor, degski's multiplier and a
+// shift; the lanes start 2^64 / the golden ratio apart (as splitmix64 counts).
 inline uint64_t key_bytes(uint64_t h, const void *p, size_t n) {
   constexpr uint64_t K = 0x9e3779b97f4a7c15ull;
   auto step = [](uint64_t a, uint64_t w) {
@@ -67,6 +68,7 @@ class LabelIndex {
   struct Entry {
     int a, b, c, k;
   };
+  // the labels times the first three 32-bit primes of xxHash
   static size_t hash(int a, int b, int c) {
     uint64_t h = ((uint64_t)(uint32_t)a * 0x9e3779b1u) ^ ((uint64_t)(uint32_t)b * 0x85ebca77u) ^ ((uint64_t)(uint32_t)c * 0xc2b2ae3du);
     return (size_t)(h ^ (h >> 15));

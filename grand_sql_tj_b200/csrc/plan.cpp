@@ -263,8 +263,9 @@ void split_tiles(const std::vector<Cell> &cells, const std::vector<Task> &tasks,
     total += k * nt;
     ntile += nt;
   }
-  // aim at tp.items_per_cta items per resident CTA (148 SMs x tp.ctas_per_sm),
-  // never below tp.min_ksteps k-steps per item
+  // aim at tp.items_per_cta items for each of 148 SMs x tp.ctas_per_sm CTAs (a
+  // count to cut for: two of the kernel's CTAs are resident on an SM), never
+  // below tp.min_ksteps k-steps per item
   const double target =
       std::max((double)tp.min_ksteps, total / (148.0 * std::max(1, tp.ctas_per_sm) * std::max(1, tp.items_per_cta)));
   // tiles in emission order with their weights; sorted below by weight,

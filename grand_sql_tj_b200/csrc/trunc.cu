@@ -545,7 +545,12 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
   // parts, one phase a step.  No buffer is doubled: a CTA sends its entries of
   // the next column once it has every CTA's parts, which each sends after its
   // last read of this column, and its next parts once it has every CTA's
-  // entries, sent after the last read of the parts before.
+  // entries, sent after the last read of the parts before.  (In the last
+  // columns a CTA may own no row from k on: it sends no entries, the others may
+  // be a step ahead of it, and their parts then count on its phase before and
+  // overwrite parts that it has not summed.  It has no use for those sums, rows
+  // of V and W to make being its only one, and over the phases the bytes are the
+  // same.)
   const uint32_t bar0 = td_smem(mbar), bar1 = td_smem(mbar + 1);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
