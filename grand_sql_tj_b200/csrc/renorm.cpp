@@ -770,7 +770,8 @@ uint64_t renorm_key(const tj_lattice *lat, int side, int mshift, const tj_model 
   h = key_bytes(h, &mshift, sizeof mshift);
   const int64_t ns = lat->num_site, ns1 = ns + 1;
   h = key_table(h, lat->neib, ns1 * lat->neibt);
-  h = key_table(h, lat->inb1, ns1 * ns1);
+  const int64_t len0 = pre->len;   // of inb1 the columns of the old and the new length are read
+  if (lat->inb1 && len0 >= 0 && len0 + 1 <= ns) h = key_table(h, lat->inb1 + len0 * ns1, 2 * ns1);
   h = key_table(h, lat->nleg11, ns);
   if (side == 1) {   // read for an environment only
     h = key_table(h, lat->nposi_dm, ns1);

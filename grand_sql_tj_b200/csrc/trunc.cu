@@ -564,9 +564,11 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
   // phases complete, as the order above asks; and whoever misses the stores (or
   // its thread 0's arrival) gives up at its own next wait, so that no mbarrier
   // meets more than two steps' bytes.
-  bool late = false;
+  // (The thread's end of the owned columns to send says so, -1 once it gave up:
+  // with a flag tested in front of the loop a step took 1 % longer.)
+  int live = nq;
   auto wait = [&](uint32_t bar, uint32_t parity) {
-    if (!late) late = !td_wait(bar, parity, limit);
+    if (live >= 0 && !td_wait(bar, parity, limit)) live = -1;
   };
   int p = 0;   // the panel's first column
   // the panel's V (below each reflector's first row), d, e and tau to global memory
@@ -748,11 +750,11 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
       __syncthreads();
     }
     // warp w sends the owned entries to CTA w
-    if (!late && warp < CL && warp != rank) {
+    if (warp < CL && warp != rank) {
       const uint32_t o = td_remote(td_smem(me), warp), ob = td_remote(bar0, warp);
-      for (int q = q0 + lane; q < nq; q += 32) td_send(o + q * 8, me[q], ob);
+      for (int q = q0 + lane; q < live; q += 32) td_send(o + q * 8, me[q], ob);
     }
-    if (!late && tid == 0) td_expect(bar0, (uint32_t)(n - k - (nq - q0)) * 8);
+    if (live >= 0 && tid == 0) td_expect(bar0, (uint32_t)(n - k - (nq - q0)) * 8);
     wait(bar0, k & 1);
     if (rank == 0 && tid == 0) de[jc] = col[k % CL * lc + k / CL];
     if (k == n - 1) break;
@@ -840,7 +842,7 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     }
     __syncthreads();
     // warp w sends the parts, and the owner of row k1 its row, to CTA w
-    if (!late && warp < CL) {
+    if (live >= 0 && warp < CL) {
       const uint32_t o = td_remote(td_smem(part + rank * TD_PL), warp), ob = td_remote(bar1, warp);
       td_send(o + lane * 8, stg[lane], ob);
       if (lane < NB) td_send(o + (2 * NB + lane) * 8, stg[2 * NB + lane], ob);
@@ -850,7 +852,7 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
         if (lane < 2) td_send(b + (2 * NB + lane) * 8, (lane ? rk : ys)[k1 / CL], ob);
       }
     }
-    if (!late && tid == 0) td_expect(bar1, (CL * TD_PT + TD_LD) * 8);
+    if (live >= 0 && tid == 0) td_expect(bar1, (CL * TD_PT + TD_LD) * 8);
     wait(bar1, k & 1);
   }
   __syncthreads();
@@ -859,7 +861,7 @@ __device__ void tridiag_coop(cg::cluster_group &cl, int rank, int s, double *Aal
     d[n - 1] = de[n - 1 - p];
     tau[n - 1] = 0.0;
   }
-  late = __syncthreads_or(late);
+  const bool late = __syncthreads_or(live < 0);
   if (late && tid == 0) atomicOr(status, 4);
   __threadfence();
   cl.sync();   // every owner's writes are visible, and no CTA sends any more
