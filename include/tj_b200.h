@@ -131,7 +131,7 @@ typedef struct tj_lattice {
  * call leaves the operator on the device and the second copies it from
  * there into data (at the DMA rate when data is page-locked); when another
  * truncation ran on the same context in between, the second call computes
- * it again. */
+ * it again, as does any call after a completed pair. */
 typedef struct tj_trunc_result {
   int32_t num_state;         /* kept states (Num_state)                             */
   int32_t num;               /* kept sectors (trun_op%num)                          */
@@ -303,7 +303,8 @@ int tj_get_hamiltonian(tj_ctx *ctx, const tj_lattice *lat, int side, int mshift,
 /* A block operator written by the library, two-call pattern as above: with
  * subs or data NULL only num and data_len are filled; then the caller
  * allocates subs[num] and data[data_len] and calls again, and `block` is
- * filled (its sub points to subs, its data to data). */
+ * filled (its sub points to subs, its data to data).  The result of a first
+ * call answers one second call; any other call computes. */
 typedef struct tj_block_result {
   int32_t num, pad_;
   int64_t data_len;
